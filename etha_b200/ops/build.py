@@ -44,7 +44,7 @@ def _fingerprint(sources: list[str], flags: list[str]) -> str:
     import hashlib
 
     h = hashlib.sha256(" ".join(flags).encode())
-    deps = sorted(sources + [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".h")])
+    deps = sorted(sources + [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh"))])
     for path in deps:
         h.update(os.path.basename(path).encode())
         with open(path, "rb") as f:

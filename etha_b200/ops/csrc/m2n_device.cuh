@@ -60,9 +60,21 @@ __device__ __forceinline__ uint4 ld_keep(const void* p) {
   return v;
 }
 
+// stores in the global state space: a plain `*p = v` could alias the op in shared memory, which would then be read again
+// after every store
 template <typename V>
 __device__ __forceinline__ void st_plain(void* p, V v) {
-  *reinterpret_cast<V*>(p) = v;
+  const size_t g = __cvta_generic_to_global(p);
+  if constexpr (sizeof(V) == 16)
+    asm volatile("st.global.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(g), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w));
+  else if constexpr (sizeof(V) == 8)
+    asm volatile("st.global.v2.u32 [%0], {%1,%2};" ::"l"(g), "r"(v.x), "r"(v.y));
+  else if constexpr (sizeof(V) == 4)
+    asm volatile("st.global.u32 [%0], %1;" ::"l"(g), "r"((uint32_t)v));
+  else if constexpr (sizeof(V) == 2)
+    asm volatile("st.global.u16 [%0], %1;" ::"l"(g), "h"((uint16_t)v));
+  else
+    asm volatile("st.global.u8 [%0], %1;" ::"l"(g), "r"((uint32_t)v));
 }
 
 // one 16-byte store delivered by NVSwitch to every GPU bound to the multicast object
@@ -227,44 +239,147 @@ __device__ __forceinline__ float round_through(float x) {
   return x;
 }
 
-// after the last CTA: publish `epoch` to every flag with system-scope release ordering
+// ---------------------------------------------------------------------------------------------
+// tile scheduling
+// ---------------------------------------------------------------------------------------------
+// The kernels are launched with one CTA per tile, and a CTA that has finished its tile takes over the tile of a CTA that
+// has not been launched yet (cluster launch control), until none is left.  Why not a grid of resident CTAs with a
+// fixed stride: SMs do not run equally fast, so fixed shares drift apart, the addresses in flight spread over many
+// DRAM pages and the slowest SM sets the end.  A bare copy of 1 GiB with 16-byte units: fixed stride 5.7 to 6.0 TB/s (read
+// + written) with any block size, unroll or cache hint; tiles taken in order as SMs become free 6.7 to 6.9; one read
+// and four writes: 5.6 and 6.6.  Why not a counter in memory: the hardware's queue belongs to the launch, so two launches of one table (two
+// streams, a graph) share nothing and nothing has to be reset.  A CTA that takes tiles over pays its prologue (and the
+// completion fence) once.
+struct TileSched {
+  uint4 handle;  // answer of try_cancel, written by the asynchronous proxy
+  uint64_t bar;
+  uint32_t op, begin, end;  // op in `s_op` and its tiles [begin, end)
+};
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void sched_init(TileSched* s) {
+  if (threadIdx.x == 0) {
+    s->op = 0xffffffffu, s->begin = 1, s->end = 0;
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&s->bar)));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+}
+
+// one thread asks for the next tile; the answer arrives while the CTA works on the present one
+__device__ __forceinline__ void sched_request(TileSched* s) {
+  const uint32_t bar = smem_addr(&s->bar);
+  asm volatile("fence.proxy.async::generic.acquire.sync_restrict::shared::cluster.cluster;" ::: "memory");
+  asm volatile("mbarrier.arrive.expect_tx.relaxed.cluster.shared::cta.b64 _, [%0], 16;" ::"r"(bar) : "memory");
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(
+                   smem_addr(&s->handle)),
+               "r"(bar)
+               : "memory");
+}
+
+// every thread waits (bounded) for the answer; returns false when no tile is left.  The caller synchronises the CTA
+// before the next request.
+__device__ __forceinline__ bool sched_take(TileSched* s, uint32_t phase, uint32_t& tile, uint32_t* sync) {
+  const uint32_t bar = smem_addr(&s->bar);
+  uint32_t ready = 0;
+  for (uint32_t spin = 0; spin < (1u << 22) && !ready; ++spin) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ready)
+        : "r"(bar), "r"(phase)
+        : "memory");
+  }
+  if (!ready) {
+    sync[1] = M2N_TIMEOUT;
+    return false;
+  }
+  uint32_t more;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b128 h;\n\t"
+      "ld.shared.b128 h, [%2];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "mov.u32 %1, 0;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, h;\n\t}"
+      : "=r"(more), "=r"(tile)
+      : "r"(smem_addr(&s->handle))
+      : "memory");
+  asm volatile("fence.proxy.async::generic.release.sync_restrict::shared::cta.cluster;" ::: "memory");
+  return more != 0;
+}
+
+// (re)load the op that owns `tile` into shared memory; the CTA is synchronised since the last use of `s_op`.  Tiles come
+// in ascending order, so the op is nearly always the one already there; otherwise warp 0 looks it up 32 ways at a time.
+__device__ __forceinline__ void sched_locate(TileSched* s, const M2NOp* __restrict__ ops,
+                                             const uint32_t* __restrict__ tile_start, uint32_t n_ops, uint32_t tile,
+                                             M2NOp* s_op) {
+  if (tile >= s->begin && tile < s->end) return;
+  __syncthreads();  // everybody has read begin / end
+  if (threadIdx.x < 32) {
+    const uint32_t lane = threadIdx.x;
+    uint32_t lo = 0, hi = n_ops;
+    while (hi - lo > 1) {
+      const uint32_t step = (hi - lo + 31) >> 5, i = lo + lane * step;
+      const uint32_t below = __ballot_sync(0xffffffffu, i < hi && tile_start[i] <= tile);
+      lo += (31 - __clz(below)) * step;
+      hi = min(hi, lo + step);
+    }
+    const uint4* g = reinterpret_cast<const uint4*>(ops + lo);
+    uint4* d = reinterpret_cast<uint4*>(s_op);
+    for (uint32_t i = lane; i < sizeof(M2NOp) / 16; i += 32) d[i] = g[i];
+    if (lane == 0) s->op = lo, s->begin = tile_start[lo], s->end = tile_start[lo + 1];
+  }
+  __syncthreads();
+}
+
+// Walk over all tiles of the table: `body(op, first unit, one past the last unit)` runs with all threads of the CTA.
+// Returns the number of tiles this CTA ran.
+template <typename Body>
+__device__ __forceinline__ uint32_t for_each_tile(TileSched* s, M2NOp* s_op, const M2NOp* __restrict__ ops,
+                                                  const uint32_t* __restrict__ tile_start, uint32_t n_ops, uint32_t* sync,
+                                                  Body&& body) {
+  sched_init(s);
+  uint32_t tile = blockIdx.x, done = 0, phase = 0;
+  while (true) {
+    if (threadIdx.x == 0) sched_request(s);
+    sched_locate(s, ops, tile_start, n_ops, tile, s_op);
+    const M2NOp& op = *s_op;
+    const uint32_t base = (tile - s->begin) * op.tile_units;
+    body(op, base, min(op.total_units, base + op.tile_units));
+    ++done;
+    const bool more = sched_take(s, phase, tile, sync);
+    phase ^= 1;
+    __syncthreads();
+    if (!more) return done;
+  }
+}
+
+// The CTA that finishes the last tile publishes `epoch` to every flag with system-scope release ordering.  Each CTA
+// releases its stores to this GPU only (fence + atomic add at GPU scope); the last one acquires all of them that way, and
+// its system-scope release stores order them for the consumers too (release patterns are cumulative).  What a small table
+// of 592 CTAs pays for its signal: 13 us with a system-scope fence in every CTA, 5 us with a GPU-scope one there and a
+// system-scope fence before the release stores, 3 us as it stands.
 __device__ __forceinline__ void finish_and_signal(uint32_t* sync, const uint64_t* signals, uint32_t n_signals,
-                                                  uint32_t epoch) {
+                                                  uint32_t epoch, uint32_t done, uint32_t total) {
   __shared__ uint32_t s_last;
   __syncthreads();
   if (threadIdx.x == 0) {
-    __threadfence_system();
-    uint32_t prev = atomicAdd(&sync[0], 1u);
-    s_last = (prev == gridDim.x - 1) ? 1u : 0u;
+    __threadfence();
+    const uint32_t prev = atomicAdd(&sync[0], done);
+    s_last = (prev + done == total) ? 1u : 0u;
+    __threadfence();
   }
   __syncthreads();
   if (s_last) {
     if (threadIdx.x == 0) sync[0] = 0;  // ready for the next launch on this stream
-    __threadfence_system();
     for (uint32_t i = threadIdx.x; i < n_signals; i += blockDim.x) {
       uint32_t* flag = reinterpret_cast<uint32_t*>(signals[i]);
       asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(flag), "r"(epoch) : "memory");
     }
   }
-}
-
-// binary search of the op that owns `tile`, and (re)load of that op into shared memory
-__device__ __forceinline__ uint32_t locate_op(const M2NOp* __restrict__ ops, const uint32_t* __restrict__ tile_start,
-                                              uint32_t n_ops, uint32_t tile, uint32_t& cur, M2NOp* s_op) {
-  uint32_t lo = 0, hi = n_ops;
-  while (hi - lo > 1) {
-    uint32_t mid = (lo + hi) >> 1;
-    if (tile_start[mid] <= tile) lo = mid; else hi = mid;
-  }
-  if (lo != cur) {
-    __syncthreads();
-    const uint4* g = reinterpret_cast<const uint4*>(ops + lo);
-    uint4* s = reinterpret_cast<uint4*>(s_op);
-    for (uint32_t i = threadIdx.x; i < sizeof(M2NOp) / 16; i += blockDim.x) s[i] = g[i];
-    __syncthreads();
-    cur = lo;
-  }
-  return lo;
 }
 
 }  // namespace

@@ -246,52 +246,87 @@ __device__ __forceinline__ bool dispatch_typed(const M2NOp& op, uint32_t base, u
 #undef CASE_RED
 }
 
-#ifndef ETHA_FAST_UNROLL
-#define ETHA_FAST_UNROLL 4
-#endif
-constexpr int kUnroll = ETHA_FAST_UNROLL;
+// Fast class: 16-byte bit copies whose box is one run or rows of a matrix (the bulk of a weight sync).  Bound by HBM (or
+// NVLink): 4 x 512 threads per SM at 30 registers, two 16-byte loads each before the first store, tiles of one such trip
+// (16 KiB).  1 GiB on one GPU, read + written: contiguous 6.57 TB/s, 2 KiB rows out of 8 KiB ones 6.38, one source and four
+// destinations 6.48 (2 x 512 threads with four loads and a fixed stride of 64 KiB tiles: 5.52, 5.79, 5.37).  With 1 KiB
+// more of spilled registers per warp the same kernel falls to 5.97, so full trips carry no per-unit predicate.
+constexpr int kFastThreads = 512;
+constexpr int kFastCtas = 4;
+constexpr int kFastUnroll = 2;
 
-// Fast class: 16-byte bit copies whose box is one run or rows of a matrix (the bulk of a weight sync).
-__global__ void __launch_bounds__(512, 2)
+// U units of one thread, kFastThreads apart, the first one `unit0`: every load is issued before the first store
+template <int ND, int U>
+__device__ __forceinline__ void fast_trip(const M2NOp& op, uint32_t unit0) {
+  uint4 v[U];
+  int64_t dof[U];
+  const char* src = reinterpret_cast<const char*>(op.src[0]);
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    if constexpr (ND == 0) {
+      dof[u] = (int64_t)unit0 * 16 + u * kFastThreads * 16;
+      v[u] = ld_stream<uint4>(src + dof[u]);
+    } else {
+      const uint32_t unit = unit0 + u * kFastThreads;
+      const uint32_t q = fast_div(unit, op.div_mul[M2N_MAX_DIMS], op.div_shr[M2N_MAX_DIMS]);
+      const uint32_t col = (unit - q * op.inner_units) * 16;
+      dof[u] = col + (int64_t)q * op.dst_stride[0];
+      v[u] = ld_stream<uint4>(src + col + (int64_t)q * op.src_stride[0]);
+    }
+  }
+  if (op.flags & M2N_FLAG_MULTIMEM) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) st_multimem16(reinterpret_cast<char*>(op.dst[0]) + dof[u], v[u]);
+    return;
+  }
+  const int nd = op.ndst;
+#pragma unroll 1
+  for (int j = 0; j < nd; ++j) {
+    char* dst = reinterpret_cast<char*>(op.dst[j]);
+#pragma unroll
+    for (int u = 0; u < U; ++u) st_plain<uint4>(dst + dof[u], v[u]);
+  }
+}
+
+template <int ND>
+__device__ __forceinline__ void fast_tile(const M2NOp& op, uint32_t base, uint32_t limit) {
+  constexpr uint32_t step = kFastThreads * kFastUnroll;
+  uint32_t b = base;
+#pragma unroll 1
+  for (; b + step <= limit; b += step) fast_trip<ND, kFastUnroll>(op, b + threadIdx.x);
+#pragma unroll 1
+  for (b += threadIdx.x; b < limit; b += kFastThreads) fast_trip<ND, 1>(op, b);
+}
+
+__global__ void __launch_bounds__(kFastThreads, kFastCtas)
 m2n_fast_kernel(const M2NOp* __restrict__ ops, const uint32_t* __restrict__ tile_start, uint32_t n_ops, uint32_t* sync,
                 const uint64_t* __restrict__ signals, uint32_t n_signals, uint32_t epoch, int do_signal) {
   __shared__ M2NOp s_op;
-  const uint32_t total_tiles = n_ops ? tile_start[n_ops] : 0;
-  uint32_t cur = 0xffffffffu;
-  for (uint32_t tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
-    const uint32_t lo = locate_op(ops, tile_start, n_ops, tile, cur, &s_op);
-    const M2NOp& op = s_op;
-    const uint32_t base = (tile - tile_start[lo]) * op.tile_units;
-    const uint32_t limit = min(op.total_units, base + op.tile_units);
-    const uint32_t step = blockDim.x * kUnroll;
-    if (op.ndim == 0) {
-      for (uint32_t b = base; b < limit; b += step) tile_raw<uint4, kUnroll, 0>(op, b, limit);
-    } else {
-      for (uint32_t b = base; b < limit; b += step) tile_raw<uint4, kUnroll, 1>(op, b, limit);
-    }
-  }
-  if (do_signal) finish_and_signal(sync, signals, n_signals, epoch);
+  __shared__ TileSched s_sched;
+  const uint32_t done = for_each_tile(&s_sched, &s_op, ops, tile_start, n_ops, sync,
+                                      [](const M2NOp& op, uint32_t base, uint32_t limit) {
+    if (op.ndim == 0) fast_tile<0>(op, base, limit);
+    else fast_tile<1>(op, base, limit);
+  });
+  if (do_signal) finish_and_signal(sync, signals, n_signals, epoch, done, gridDim.x);
 }
 
 // General class: any other bit copy, converting copies and Partial collapses.
+constexpr int kGeneralThreads = 256;
 constexpr int kGenUnroll = 2;
 template <typename V>
 __device__ __noinline__ void walk_raw(const M2NOp& op, uint32_t base, uint32_t limit) {
   for (uint32_t b = base; b < limit; b += blockDim.x * kGenUnroll) tile_raw<V, kGenUnroll, -1>(op, b, limit);
 }
 
-__global__ void __launch_bounds__(256, ETHA_GENERAL_CTAS)
+__global__ void __launch_bounds__(kGeneralThreads, ETHA_GENERAL_CTAS)
 m2n_general_kernel(const M2NOp* __restrict__ ops, const uint32_t* __restrict__ tile_start, uint32_t n_ops,
                    uint32_t* sync, const uint64_t* __restrict__ signals, uint32_t n_signals, uint32_t epoch,
                    int do_signal) {
   __shared__ M2NOp s_op;
-  const uint32_t total_tiles = n_ops ? tile_start[n_ops] : 0;
-  uint32_t cur = 0xffffffffu;
-  for (uint32_t tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
-    const uint32_t lo = locate_op(ops, tile_start, n_ops, tile, cur, &s_op);
-    const M2NOp& op = s_op;
-    const uint32_t base = (tile - tile_start[lo]) * op.tile_units;
-    const uint32_t limit = min(op.total_units, base + op.tile_units);
+  __shared__ TileSched s_sched;
+  const uint32_t done = for_each_tile(&s_sched, &s_op, ops, tile_start, n_ops, sync,
+                                      [sync](const M2NOp& op, uint32_t base, uint32_t limit) {
     if (op.mode == M2N_MODE_RAW) {
       switch (op.unit_bytes_src) {
         case 16: walk_raw<uint4>(op, base, limit); break;
@@ -303,8 +338,8 @@ m2n_general_kernel(const M2NOp* __restrict__ ops, const uint32_t* __restrict__ t
     } else if (!dispatch_typed(op, base, limit)) {
       if (threadIdx.x == 0) sync[1] = M2N_BAD_OP;
     }
-  }
-  if (do_signal) finish_and_signal(sync, signals, n_signals, epoch);
+  });
+  if (do_signal) finish_and_signal(sync, signals, n_signals, epoch, done, gridDim.x);
 }
 
 __global__ void set_flags_kernel(const uint64_t* __restrict__ signals, uint32_t n_signals, uint32_t epoch) {
@@ -357,21 +392,24 @@ inline int fail(cudaError_t e, const char* what) {
 
 extern "C" {
 
-// resident 256-thread CTAs per SM the general kernel was compiled for (the launcher sizes its grid with it)
-int etha_general_ctas_per_sm(void) { return ETHA_GENERAL_CTAS; }
-
-int etha_m2n_launch(const M2NOp* ops, const uint32_t* tile_start, uint32_t n_ops, int typed, int grid, int block,
-                    uint32_t* sync_scratch, const uint64_t* signals, uint32_t n_signals, uint32_t epoch,
+int etha_m2n_launch(const M2NOp* ops, const uint32_t* tile_start, uint32_t n_ops, int general, uint32_t n_tiles,
+                    int ctas_per_sm, uint32_t* sync_scratch, const uint64_t* signals, uint32_t n_signals, uint32_t epoch,
                     int do_signal, void* stream) {
-  if (grid < 1) grid = 1;
-  if (typed) {
-    if (block < 32 || block > 256 || (block & 31)) block = 256;
-    m2n_general_kernel<<<grid, block, 0, (cudaStream_t)stream>>>(ops, tile_start, n_ops, sync_scratch, signals, n_signals,
-                                                               epoch, do_signal);
+  if (!n_tiles) return 0;
+  cudaStream_t s = (cudaStream_t)stream;
+  if (general) {
+    m2n_general_kernel<<<n_tiles, kGeneralThreads, 0, s>>>(ops, tile_start, n_ops, sync_scratch, signals, n_signals, epoch,
+                                                           do_signal);
   } else {
-    if (block < 32 || block > 512 || (block & 31)) block = 512;
-    m2n_fast_kernel<<<grid, block, 0, (cudaStream_t)stream>>>(ops, tile_start, n_ops, sync_scratch, signals, n_signals,
-                                                             epoch, do_signal);
+    // a caller that asks for one CTA per SM (of the two that fill it by default) leaves half of each SM to other work:
+    // shared memory that is never touched lets two of the four CTAs in
+    const int smem = ctas_per_sm == 1 ? 76 * 1024 : 0;
+    if (smem) {
+      cudaError_t e = cudaFuncSetAttribute(m2n_fast_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+      if (e != cudaSuccess) return fail(e, "fast kernel shared memory opt-in");
+    }
+    m2n_fast_kernel<<<n_tiles, kFastThreads, smem, s>>>(ops, tile_start, n_ops, sync_scratch, signals, n_signals, epoch,
+                                                        do_signal);
   }
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : fail(e, "m2n kernel launch");
@@ -413,11 +451,10 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[ETHA_NOALLOC_SC
 constexpr int kMaxDevices = 64;
 std::mutex g_noalloc_mu;
 unsigned char* g_noalloc_ptr[kMaxDevices] = {nullptr};
-int g_noalloc_sms[kMaxDevices] = {0};
 
 // Host code must not use `g_noalloc_scratch` as an address: there it is only a stand-in for the symbol.
 // The device address is queried once per device, with that device current.
-int noalloc_setup(int dev, unsigned char** out, int* sms) {
+int noalloc_setup(int dev, unsigned char** out) {
   std::lock_guard<std::mutex> lock(g_noalloc_mu);
   if (dev < 0 || dev >= kMaxDevices) {
     snprintf(etha_err_buf(), ETHA_ERR_LEN, "device index %d out of range", dev);
@@ -427,14 +464,9 @@ int noalloc_setup(int dev, unsigned char** out, int* sms) {
     void* p = nullptr;
     cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
     if (e != cudaSuccess || !p) return fail(e, "cudaGetSymbolAddress(scratch)");
-    int n = 0;
-    e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return fail(e, "cudaDeviceGetAttribute(sm count)");
-    g_noalloc_sms[dev] = n;
     g_noalloc_ptr[dev] = static_cast<unsigned char*>(p);
   }
   *out = g_noalloc_ptr[dev];
-  *sms = g_noalloc_sms[dev];
   return 0;
 }
 
@@ -443,6 +475,7 @@ int noalloc_setup(int dev, unsigned char** out, int* sms) {
 extern "C" int etha_pack_op(const M2NOpSpec* spec, M2NOp* out, char* err, int err_len);
 extern "C" uint32_t etha_op_tiles(const M2NOp* op);
 extern "C" int etha_op_class(const M2NOp* op);
+extern "C" int64_t etha_layout_tiles(M2NOp* ops, uint32_t n_ops, int kernel, uint32_t* tile_start);
 
 extern "C" int etha_m2n_run_noalloc(const M2NOpSpec* specs, uint32_t n_specs, int ctas_per_sm, void* stream) {
   if (!specs && n_specs) {
@@ -467,30 +500,26 @@ extern "C" int etha_m2n_run_noalloc(const M2NOpSpec* specs, uint32_t n_specs, in
     return -101;
   }
   unsigned char* scratch = nullptr;
-  int sms = 0;
-  int rc = noalloc_setup(dev, &scratch, &sms);
+  int rc = noalloc_setup(dev, &scratch);
   if (rc != 0) return rc;
 
   // host staging lives in thread-local storage: no heap allocation per call
   static thread_local M2NOp packed[2][ETHA_NOALLOC_MAX_OPS];
   static thread_local uint32_t tile_start[2][ETHA_NOALLOC_MAX_OPS + 1];
   uint32_t count[2] = {0, 0};
-  tile_start[0][0] = tile_start[1][0] = 0;
   for (uint32_t i = 0; i < n_specs; ++i) {
     M2NOp op;
     rc = etha_pack_op(&specs[i], &op, etha_err_buf(), ETHA_ERR_LEN);
     if (rc != 0) return rc;
-    const uint32_t tiles = etha_op_tiles(&op);
-    if (!tiles) continue;
+    if (!etha_op_tiles(&op)) continue;
     const int c = etha_op_class(&op);
-    const uint64_t next = (uint64_t)tile_start[c][count[c]] + tiles;
-    if (next >= (1ull << 32)) {
+    packed[c][count[c]++] = op;
+  }
+  for (int c = 0; c < 2; ++c)
+    if (etha_layout_tiles(packed[c], count[c], c, tile_start[c]) < 0) {
       snprintf(etha_err_buf(), ETHA_ERR_LEN, "too many tiles in one call");
       return -101;
     }
-    packed[c][count[c]] = op;
-    tile_start[c][++count[c]] = (uint32_t)next;
-  }
   cudaStream_t s = (cudaStream_t)stream;
   // counters must start at zero whatever the previous call left there
   e = cudaMemsetAsync(scratch, 0, 512, s);
@@ -505,16 +534,9 @@ extern "C" int etha_m2n_run_noalloc(const M2NOpSpec* specs, uint32_t n_specs, in
     if (e != cudaSuccess) return fail(e, "cudaMemcpyAsync(tile table)");
     e = cudaMemcpyAsync(class_ops, packed[c], count[c] * sizeof(M2NOp), cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) return fail(e, "cudaMemcpyAsync(op table)");
-    const uint32_t total = tile_start[c][count[c]];
-    int grid = (int)(total < (uint32_t)(sms * ctas_per_sm) ? total : (uint32_t)(sms * ctas_per_sm));
-    if (grid < 1) grid = 1;
     uint32_t* sync = reinterpret_cast<uint32_t*>(scratch + 256 * c);
-    if (c == 0)
-      m2n_fast_kernel<<<grid, 512, 0, s>>>(class_ops, tiles_dev, count[c], sync, nullptr, 0, 0, 0);
-    else
-      m2n_general_kernel<<<grid, 256, 0, s>>>(class_ops, tiles_dev, count[c], sync, nullptr, 0, 0, 0);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return fail(e, "allocation-free launch");
+    rc = etha_m2n_launch(class_ops, tiles_dev, count[c], c, tile_start[c][count[c]], ctas_per_sm, sync, nullptr, 0, 0, 0, s);
+    if (rc != 0) return rc;
   }
   return 0;
 }
@@ -524,8 +546,7 @@ extern "C" int etha_m2n_noalloc_status(uint32_t* status, void* stream) {
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return fail(e, "cudaGetDevice");
   unsigned char* scratch = nullptr;
-  int sms = 0;
-  int rc = noalloc_setup(dev, &scratch, &sms);
+  int rc = noalloc_setup(dev, &scratch);
   if (rc != 0) return rc;
   uint32_t words[2] = {0, 0};
   e = cudaMemcpyAsync(&words[0], scratch + 4, 4, cudaMemcpyDeviceToHost, (cudaStream_t)stream);

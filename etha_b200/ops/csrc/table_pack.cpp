@@ -60,6 +60,28 @@ uint32_t etha_op_tiles(const M2NOp* op) {
   return (op->total_units + op->tile_units - 1) / op->tile_units;
 }
 
+// Tile sizes.  A large table gets tiles of one trip of the kernel's loads (1024 units for the fast and the streaming
+// kernels, eight trips of the general kernel: 4096 units run a two-byte ragged copy in 139 us, 1024 units in 158): CTAs take tiles in order as they become free, so small tiles keep the
+// addresses in flight together and the end even.  Copy of 1 GiB with 16-byte units: 8 KiB tiles (half the threads idle)
+// 5.81 TB/s, 16 KiB 6.57, 32 KiB 6.51, 64 KiB 6.37; one source and four destinations: 6.61, 6.48, 6.26, 6.11.  A table too small for that is spread over all CTAs the chip holds, down to one unit per
+// thread of a 256-thread block: a 3.4 MB model took 11.8 us as 60 tiles of 64 KiB.
+int64_t etha_layout_tiles(M2NOp* ops, uint32_t n_ops, int kernel, uint32_t* tile_start) {
+  const uint32_t max_units = kernel == 1 ? 4096 : 1024, min_units = 256;
+  const uint64_t ctas = 148 * 4;
+  uint64_t total = 0, tiles = 0;
+  for (uint32_t i = 0; i < n_ops; ++i) total += ops[i].total_units;
+  const uint64_t share = (total + ctas - 1) / ctas;
+  const uint64_t units = std::min<uint64_t>(max_units, std::max<uint64_t>(min_units, (share + 255) / 256 * 256));
+  tile_start[0] = 0;
+  for (uint32_t i = 0; i < n_ops; ++i) {
+    ops[i].tile_units = (uint32_t)std::min<uint64_t>(units, ops[i].tile_units);
+    tiles += etha_op_tiles(&ops[i]);
+    if (tiles >= (1ull << 31)) return -1;  // a grid holds fewer
+    tile_start[i + 1] = (uint32_t)tiles;
+  }
+  return (int64_t)tiles;
+}
+
 int etha_pack_op(const M2NOpSpec* s, M2NOp* o, char* err, int err_len) {
   memset(o, 0, sizeof(*o));
   if (s->ndim < 0 || s->ndim > 8) return error(err, err_len, -1, "ndim %d out of range", s->ndim);

@@ -69,7 +69,8 @@ def cuda_lib() -> C.CDLL:
         lib.etha_op_tiles.restype = u32
         lib.etha_op_class.argtypes = [vp]
         lib.etha_op_class.restype = i32
-        lib.etha_general_ctas_per_sm.restype = i32
+        lib.etha_layout_tiles.argtypes = [vp, u32, i32, vp]
+        lib.etha_layout_tiles.restype = C.c_int64
         lib.etha_op_bulk_ok.argtypes = [vp]
         lib.etha_op_bulk_ok.restype = i32
         lib.etha_m2n_run_noalloc.argtypes = [C.POINTER(OpSpec), u32, i32, vp]
@@ -78,10 +79,9 @@ def cuda_lib() -> C.CDLL:
         lib.etha_m2n_noalloc_status.restype = i32
         lib.etha_op_stream_key.argtypes = [vp]
         lib.etha_op_stream_key.restype = i32
-        lib.etha_stream_ctas_per_sm.restype = i32
-        lib.etha_m2n_typed_launch.argtypes = [vp, vp, u32, i32, i32, vp, vp, u32, u32, i32, vp]
+        lib.etha_m2n_typed_launch.argtypes = [vp, vp, u32, i32, u32, vp, vp, u32, u32, i32, vp]
         lib.etha_m2n_typed_launch.restype = i32
-        lib.etha_m2n_launch.argtypes = [vp, vp, u32, i32, i32, i32, vp, vp, u32, u32, i32, vp]
+        lib.etha_m2n_launch.argtypes = [vp, vp, u32, i32, u32, i32, vp, vp, u32, u32, i32, vp]
         lib.etha_m2n_launch.restype = i32
         lib.etha_set_flags.argtypes = [vp, u32, u32, vp]
         lib.etha_set_flags.restype = i32
@@ -110,7 +110,7 @@ def cuda_lib() -> C.CDLL:
         lib.etha_device_info.argtypes = [C.POINTER(i32)] * 4
         lib.etha_device_info.restype = i32
         if hasattr(lib, "etha_m2n_bulk_launch"):
-            lib.etha_m2n_bulk_launch.argtypes = [vp, vp, u32, i32, vp, vp, u32, u32, i32, vp]
+            lib.etha_m2n_bulk_launch.argtypes = [vp, vp, u32, u32, vp, vp, u32, u32, i32, vp]
             lib.etha_m2n_bulk_launch.restype = i32
         _lib = lib
         return lib

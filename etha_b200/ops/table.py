@@ -53,16 +53,40 @@ class SliceRef:
 
 
 class _KernelSet:
-    """Device arrays of the kernel classes for one set of ops."""
+    """Launches that run one set of ops: `[(kernel, ops address, tile table address, number of ops, tiles), ...]`, without
+    and with the TMA kernel.  Until the table is uploaded the addresses are offsets into its buffer."""
 
     def __init__(self):
-        self.ops_dev: list[torch.Tensor | None] = [None, None]
-        self.tiles_dev: list[torch.Tensor | None] = [None, None]
-        self.tiles_rest_dev: torch.Tensor | None = None  # prefix sums of the fast ops the TMA kernel cannot run
-        self.n_ops, self.n_tiles = [0, 0], [0, 0]
+        self.n_ops, self.n_tiles = [0, 0], [0, 0]  # [fast class, general class]
+        self.n_typed_ops = self.n_typed_tiles = 0
         self.n_bulk_ops = self.n_bulk_tiles = 0
-        # streaming instances of the typed class: key -> (ops, tile prefix sums, number of ops, tiles)
-        self.typed: dict[int, tuple[torch.Tensor, torch.Tensor, int, int]] = {}
+        self.ldst: list[tuple] = []
+        self.bulk: list[tuple] = []
+
+    def at(self, base: int) -> "_KernelSet":
+        for name in ("ldst", "bulk"):
+            setattr(self, name, [(k, base + ops, base + tiles, n, t) for k, ops, tiles, n, t in getattr(self, name)])
+        return self
+
+
+class _Blob:
+    """Host image of everything a table keeps on the device, uploaded in one copy."""
+
+    def __init__(self):
+        self.parts: list[tuple[int, np.ndarray]] = []
+        self.size = 0
+
+    def add(self, array: np.ndarray) -> int:
+        offset = (self.size + 15) // 16 * 16
+        self.parts.append((offset, array))
+        self.size = offset + array.nbytes
+        return offset
+
+    def upload(self, device) -> torch.Tensor:
+        image = np.zeros(self.size, dtype=np.uint8)
+        for offset, array in self.parts:
+            image[offset : offset + array.nbytes] = array.view(np.uint8)
+        return torch.from_numpy(image).to(device)
 
 
 class CopyTable:
@@ -190,42 +214,49 @@ class CopyTable:
         self.add(tuple(dst.shape), [SliceRef.of(s) for s in srcs], [SliceRef.of(dst)], sizes, ops)
 
     # ---- upload -----------------------------------------------------------------------------
-    def _upload(self, packed) -> "_KernelSet":
-        """Device arrays of one set of packed ops, split into the kernel classes."""
+    def _lay_out(self, packed, blob: _Blob) -> "_KernelSet":
+        """Put one set of packed ops into `blob`, split into the launches of the kernel classes."""
         ks = _KernelSet()
 
-        def prefix(tiles):
-            starts = np.zeros(len(tiles) + 1, dtype=np.uint64)
-            np.cumsum(tiles, out=starts[1:])
-            if starts[-1] >= 2**32:
+        def launch(kernel, members, tile_class):
+            """One launch: tile sizes chosen for its kernel."""
+            ops_host = np.frombuffer(b"".join(members), dtype=np.uint8).copy()
+            starts = np.zeros(len(members) + 1, dtype=np.uint32)
+            tiles = self._lib.etha_layout_tiles(ops_host.ctypes.data, len(members), tile_class, starts.ctypes.data)
+            if tiles < 0:
                 raise ValueError("too many tiles in one table")
-            return starts
+            return kernel, blob.add(ops_host), blob.add(starts), len(members), tiles
 
-        def to_dev(starts):
-            return torch.from_numpy(starts.astype(np.uint32).view(np.int32).copy()).to(self.device)
-
-        keys = list(dict.fromkeys(k for c, _, _, _, k in packed if c == 1 and k))
-        for key in keys:
-            members = [(t, raw) for c, t, raw, _, k in packed if c == 1 and k == key]
-            starts = prefix([t for t, _ in members])
-            blob = np.frombuffer(b"".join(raw for _, raw in members), dtype=np.uint8)
-            ks.typed[key] = (torch.from_numpy(blob.copy()).to(self.device), to_dev(starts), len(members), int(starts[-1]))
-        for cls in (0, 1):
-            members = [(t, raw, tma) for c, t, raw, tma, k in packed if c == cls and not (c == 1 and k)]
-            if cls == 0:  # stable split: TMA-capable ops first, relative order kept inside both groups
-                members = [m for m in members if m[2]] + [m for m in members if not m[2]]
-                ks.n_bulk_ops = sum(1 for m in members if m[2])
-                ks.n_bulk_tiles = sum(m[0] for m in members if m[2])
-            ks.n_ops[cls] = len(members)
-            if not members:
-                continue
-            starts = prefix([t for t, _, _ in members])
-            ks.n_tiles[cls] = int(starts[-1])
-            blob = np.frombuffer(b"".join(raw for _, raw, _ in members), dtype=np.uint8)
-            ks.ops_dev[cls] = torch.from_numpy(blob.copy()).to(self.device)
-            ks.tiles_dev[cls] = to_dev(starts)
-            if cls == 0 and 0 < ks.n_bulk_ops < len(members):
-                ks.tiles_rest_dev = to_dev(prefix([t for t, _, _ in members[ks.n_bulk_ops:]]))
+        rest = []  # launches of the typed and general classes
+        for key in dict.fromkeys(k for c, _, _, _, k in packed if c == 1 and k):
+            rest.append(launch(key, [raw for c, _, raw, _, k in packed if c == 1 and k == key], 0))
+            ks.n_typed_ops += rest[-1][3]
+            ks.n_typed_tiles += rest[-1][4]
+        general = [raw for c, _, raw, _, k in packed if c == 1 and not k]
+        if general:
+            rest.append(launch("general", general, 1))
+            ks.n_ops[1], ks.n_tiles[1] = rest[-1][3:]
+        fast = [(t, raw, tma) for c, t, raw, tma, _ in packed if c == 0]
+        if fast:
+            # stable split: TMA-capable ops first, relative order kept inside both groups
+            tma, other = [m for m in fast if m[2]], [m for m in fast if not m[2]]
+            ks.ldst.append(launch("fast", [raw for _, raw, _ in tma + other], 0))
+            ks.n_ops[0], ks.n_tiles[0] = ks.ldst[0][3:]
+            if tma:
+                # the TMA kernel cuts its tiles into ring stages and keeps the table's tile size
+                starts = np.zeros(len(tma) + 1, dtype=np.uint64)
+                np.cumsum([t for t, _, _ in tma], out=starts[1:])
+                if starts[-1] >= 2**31:
+                    raise ValueError("too many tiles in one table")
+                ks.n_bulk_ops, ks.n_bulk_tiles = len(tma), int(starts[-1])
+                ks.bulk.append(("bulk", blob.add(np.frombuffer(b"".join(raw for _, raw, _ in tma), dtype=np.uint8)),
+                                blob.add(starts.astype(np.uint32)), len(tma), ks.n_bulk_tiles))
+                if other:
+                    ks.bulk.append(launch("fast", [raw for _, raw, _ in other], 0))
+            else:
+                ks.bulk = list(ks.ldst)
+        ks.ldst += rest
+        ks.bulk += rest
         return ks
 
     def _select_dma(self) -> set[int]:
@@ -251,18 +282,21 @@ class CopyTable:
             sm_count = torch.cuda.get_device_properties(self.device).multi_processor_count
         self.sm_count = sm_count
         taken = self._select_dma()
+        blob = _Blob()
+        blob.add(np.zeros(4, dtype=np.uint32))  # finished tiles and error word of the launches
         # two kernel sets share this table: every op (kernels only), and what is left next to the DMA copies
-        self._all = self._upload(self._packed)
-        self._rest = self._upload([e for i, e in enumerate(self._packed) if i not in taken]) if taken else self._all
-        typed_ops = sum(v[2] for v in self._all.typed.values())
-        typed_tiles = sum(v[3] for v in self._all.typed.values())
+        self._all = self._lay_out(self._packed, blob)
+        self._rest = self._lay_out([e for i, e in enumerate(self._packed) if i not in taken], blob) if taken else self._all
+        self._buffer = blob.upload(self.device)
+        self._sync = self._buffer[:16].view(torch.int32)
+        for ks in {id(k): k for k in (self._all, self._rest)}.values():
+            ks.at(self._buffer.data_ptr())
         # [fast class, typed + general]: the streaming instances count with the general class they were taken from
-        self.n_ops = [self._all.n_ops[0], self._all.n_ops[1] + typed_ops]
-        self.n_tiles = [self._all.n_tiles[0], self._all.n_tiles[1] + typed_tiles]
-        self.n_typed_ops = typed_ops
+        self.n_ops = [self._all.n_ops[0], self._all.n_ops[1] + self._all.n_typed_ops]
+        self.n_tiles = [self._all.n_tiles[0], self._all.n_tiles[1] + self._all.n_typed_tiles]
+        self.n_typed_ops = self._all.n_typed_ops
         self.n_bulk_ops, self.n_bulk_tiles = self._all.n_bulk_ops, self._all.n_bulk_tiles
         self._dma_candidates = []
-        self._sync = torch.zeros(4, dtype=torch.int32, device=self.device)
         self._packed = []
         if self._dma:
             arr = (L.DmaCopy * len(self._dma))(*self._dma)
@@ -291,13 +325,8 @@ class CopyTable:
         return self.n_tiles[0] + self.n_tiles[1] == 0
 
     def device_buffers(self) -> list[torch.Tensor]:
-        """Every device array a launch reads (callers that drop the table right after a launch tie these to the stream)."""
-        out = [self._sync]
-        for ks in {id(self._all): self._all, id(self._rest): self._rest}.values():
-            out += [b for b in (*ks.ops_dev, *ks.tiles_dev, ks.tiles_rest_dev) if b is not None]
-            for ops_t, tiles_t, _, _ in ks.typed.values():
-                out += [ops_t, tiles_t]
-        return out
+        """The device memory a launch reads (callers that drop the table right after a launch tie it to the stream)."""
+        return [self._buffer]
 
     # ---- launch -----------------------------------------------------------------------------
     def launch(
@@ -319,22 +348,7 @@ class CopyTable:
         sig_ptr = 0 if signals is None else signals.data_ptr()
         dma = self._dma_plan is not None and dma is not False
         ks = self._rest if dma else self._all
-        # launches of this transfer: (kernel, ops, tile prefix sums, number of ops, tiles)
-        plan = []
-        if ks.n_tiles[0]:
-            ops0, tiles0 = ks.ops_dev[0].data_ptr(), ks.tiles_dev[0].data_ptr()
-            if bulk and ks.n_bulk_tiles:
-                plan.append(("bulk", ops0, tiles0, ks.n_bulk_ops, ks.n_bulk_tiles))
-                rest = ks.n_ops[0] - ks.n_bulk_ops
-                if rest:
-                    plan.append(("fast", ops0 + ks.n_bulk_ops * self._op_size, ks.tiles_rest_dev.data_ptr(), rest,
-                                 ks.n_tiles[0] - ks.n_bulk_tiles))
-            else:
-                plan.append(("fast", ops0, tiles0, ks.n_ops[0], ks.n_tiles[0]))
-        for key, (ops_t, tiles_t, n, tiles) in ks.typed.items():
-            plan.append((key, ops_t.data_ptr(), tiles_t.data_ptr(), n, tiles))
-        if ks.n_tiles[1]:
-            plan.append(("general", ks.ops_dev[1].data_ptr(), ks.tiles_dev[1].data_ptr(), ks.n_ops[1], ks.n_tiles[1]))
+        plan = ks.bulk if bulk else ks.ldst
         if not plan or dma:
             # with DMA copies in the transfer: the copies start on side streams, the kernels run next to them on
             # the caller's stream without a signal, the stream then waits for the copies and the flags go last
@@ -356,16 +370,11 @@ class CopyTable:
 
     def _launch_kernel(self, kernel, ops_ptr, tiles_ptr, n_ops, n_tiles, ctas_per_sm, sig, s) -> None:
         if kernel == "bulk":
-            rc = self._lib.etha_m2n_bulk_launch(ops_ptr, tiles_ptr, n_ops, min(n_tiles, self.sm_count),
-                                                self._sync.data_ptr(), *sig, s)
+            rc = self._lib.etha_m2n_bulk_launch(ops_ptr, tiles_ptr, n_ops, n_tiles, self._sync.data_ptr(), *sig, s)
         elif isinstance(kernel, int):  # key of a streaming instance
-            grid = min(n_tiles, self.sm_count * self._lib.etha_stream_ctas_per_sm())
-            rc = self._lib.etha_m2n_typed_launch(ops_ptr, tiles_ptr, n_ops, kernel, grid, self._sync.data_ptr(), *sig, s)
+            rc = self._lib.etha_m2n_typed_launch(ops_ptr, tiles_ptr, n_ops, kernel, n_tiles, self._sync.data_ptr(), *sig, s)
         else:
-            general = kernel == "general"
-            # the fast kernel is compiled for two 512-thread CTAs per SM; the general one reports its own occupancy
-            per_sm = max(ctas_per_sm, self._lib.etha_general_ctas_per_sm()) if general else ctas_per_sm
-            rc = self._lib.etha_m2n_launch(ops_ptr, tiles_ptr, n_ops, int(general), min(n_tiles, self.sm_count * per_sm), 0,
+            rc = self._lib.etha_m2n_launch(ops_ptr, tiles_ptr, n_ops, int(kernel == "general"), n_tiles, ctas_per_sm,
                                            self._sync.data_ptr(), *sig, s)
         L.check(rc, "m2n launch")
         LAUNCH_COUNT[0] += 1
