@@ -336,8 +336,8 @@ __device__ __forceinline__ void sched_locate(TileSched* s, const M2NOp* __restri
 }
 
 // Walk over all tiles of the table: `body(op, first unit, one past the last unit)` runs with all threads of the CTA.
-// Returns the number of tiles this CTA ran.
-template <typename Body>
+// Returns the number of tiles this CTA ran.  CHUNKS: the tiles are counted in the op's chunks instead of its units.
+template <bool CHUNKS = false, typename Body>
 __device__ __forceinline__ uint32_t for_each_tile(TileSched* s, M2NOp* s_op, const M2NOp* __restrict__ ops,
                                                   const uint32_t* __restrict__ tile_start, uint32_t n_ops, uint32_t* sync,
                                                   Body&& body) {
@@ -348,7 +348,7 @@ __device__ __forceinline__ uint32_t for_each_tile(TileSched* s, M2NOp* s_op, con
     sched_locate(s, ops, tile_start, n_ops, tile, s_op);
     const M2NOp& op = *s_op;
     const uint32_t base = (tile - s->begin) * op.tile_units;
-    body(op, base, min(op.total_units, base + op.tile_units));
+    body(op, base, min(CHUNKS ? op.chunks : op.total_units, base + op.tile_units));
     ++done;
     const bool more = sched_take(s, phase, tile, sync);
     phase ^= 1;

@@ -69,13 +69,14 @@ int64_t etha_layout_tiles(M2NOp* ops, uint32_t n_ops, int kernel, uint32_t* tile
   const uint32_t max_units = kernel == 1 ? 4096 : 1024, min_units = 256;
   const uint64_t ctas = 148 * 4;
   uint64_t total = 0, tiles = 0;
-  for (uint32_t i = 0; i < n_ops; ++i) total += ops[i].total_units;
+  const auto count = [&](const M2NOp& op) { return kernel == 2 ? op.chunks : op.total_units; };
+  for (uint32_t i = 0; i < n_ops; ++i) total += count(ops[i]);
   const uint64_t share = (total + ctas - 1) / ctas;
   const uint64_t units = std::min<uint64_t>(max_units, std::max<uint64_t>(min_units, (share + 255) / 256 * 256));
   tile_start[0] = 0;
   for (uint32_t i = 0; i < n_ops; ++i) {
     ops[i].tile_units = (uint32_t)std::min<uint64_t>(units, ops[i].tile_units);
-    tiles += etha_op_tiles(&ops[i]);
+    tiles += (count(ops[i]) + ops[i].tile_units - 1) / ops[i].tile_units;
     if (tiles >= (1ull << 31)) return -1;  // a grid holds fewer
     tile_start[i + 1] = (uint32_t)tiles;
   }
@@ -220,6 +221,39 @@ int etha_pack_op(const M2NOpSpec* s, M2NOp* o, char* err, int err_len) {
   int64_t tu = (tile_bytes + ubd - 1) / ubd;
   tu = ((tu + 2047) / 2048) * 2048;
   o->tile_units = (uint32_t)std::min<int64_t>(tu, 1ll << 30);
+
+  // Ragged class: rows that are runs on both sides, in units below the widest ones or with two or more strided dims.
+  // Shorter rows than 48 bytes have more partial than whole chunks and stay element-wise.  The destinations of a fan-out
+  // must agree on where the 16-byte boundaries are.
+  const bool widest = mode == M2N_MODE_RAW ? ubs == 16 : unit_elems == 8;
+  const int64_t row_bytes = inner_elems * ed, row_src_bytes = inner_elems * es;
+  bool ragged = (!widest || dims.size() > 1) && !(s->flags & M2N_FLAG_MULTIMEM) && row_bytes >= 48 && row_src_bytes >= 48 &&
+                row_bytes < (1ll << 30) && row_src_bytes < (1ll << 30);
+  for (int i = 1; i < s->ndst; ++i) ragged = ragged && (s->dst[i] & 15) == (s->dst[0] & 15);
+  if (mode != M2N_MODE_RAW) {  // elements on their natural boundaries
+    for (int i = 0; i < s->ndst; ++i) ragged = ragged && s->dst[i] % ed == 0;
+    for (int i = 0; i < s->nsrc; ++i) ragged = ragged && s->src[i] % es == 0;
+  }
+  if (ragged) {
+    // a row has one chunk more than its bytes need wherever its first chunk is partial; the offset is the same for every
+    // row if the strides are multiples of 16 bytes
+    bool fixed = true;
+    for (auto& d : dims) fixed = fixed && (d.ds * ed) % 16 == 0;
+    const int64_t per = mode == M2N_MODE_RAW ? M2N_RAGGED_BYTES : 8, len = mode == M2N_MODE_RAW ? row_bytes : inner_elems;
+    int64_t lead = mode == M2N_MODE_RAW ? 15 : 7;
+    if (fixed && mode == M2N_MODE_RAW) {
+      lead = (int64_t)(s->dst[0] & 15);
+    } else if (fixed) {
+      const int64_t head = (int64_t)((0 - s->dst[0]) & 15) / ed;
+      lead = head ? 8 - head : 0;
+    }
+    const int64_t per_row = (len + lead + per - 1) / per, all = total / inner_units * per_row;
+    if (all < (1ll << 31)) {
+      o->chunks = (uint32_t)all;
+      o->chunk_row = (uint32_t)per_row;
+      magic((uint32_t)per_row, &o->chunk_mul, &o->chunk_shr);
+    }
+  }
   return 0;
 }
 

@@ -111,8 +111,9 @@ class CopyTable:
         self.dma_bytes = 0
         self._lib = L.cuda_lib()
         self._op_size = self._lib.etha_sizeof_op()
-        self._packed: list[tuple[int, int, bytes, bool, int]] = []  # (class, tiles, op bytes, TMA-capable, stream key)
-        self.stream_typed = True  # conversions / collapses over simple boxes use the streaming kernel instances
+        self._packed: list[tuple[int, int, bytes, bool, int]] = []  # (class, tiles, op bytes, TMA-capable, instance key)
+        # conversions / collapses over simple boxes use the streaming kernel instances, rows of any alignment the ragged ones
+        self.stream_typed = True
         self.payload_bytes = 0  # bytes delivered (destination side, all replicas)
         self.read_bytes = 0
         self._final = False
@@ -186,7 +187,9 @@ class CopyTable:
                 if tiles:
                     cls = self._lib.etha_op_class(buf)
                     tma = cls == 0 and bool(self._lib.etha_op_bulk_ok(buf))
-                    skey = self._lib.etha_op_stream_key(buf) if (cls == 1 and self.stream_typed) else 0
+                    skey = 0
+                    if cls == 1 and self.stream_typed:
+                        skey = self._lib.etha_op_stream_key(buf) or self._lib.etha_op_ragged_key(buf)
                     entry = (cls, tiles, buf.raw, tma, skey)
                     self._packed.append(entry)
                     if dma_ok and self.dma_min_bytes is not None and numel * ddtype.itemsize >= self.dma_min_bytes:
@@ -229,13 +232,19 @@ class CopyTable:
 
         rest = []  # launches of the typed and general classes
         for key in dict.fromkeys(k for c, _, _, _, k in packed if c == 1 and k):
-            rest.append(launch(key, [raw for c, _, raw, _, k in packed if c == 1 and k == key], 0))
-            ks.n_typed_ops += rest[-1][3]
-            ks.n_typed_tiles += rest[-1][4]
+            ragged = key >= L.KEY_RAGGED
+            rest.append(launch(key, [raw for c, _, raw, _, k in packed if c == 1 and k == key], 2 if ragged else 0))
+            if ragged:
+                ks.n_ops[1] += rest[-1][3]
+                ks.n_tiles[1] += rest[-1][4]
+            else:
+                ks.n_typed_ops += rest[-1][3]
+                ks.n_typed_tiles += rest[-1][4]
         general = [raw for c, _, raw, _, k in packed if c == 1 and not k]
         if general:
             rest.append(launch("general", general, 1))
-            ks.n_ops[1], ks.n_tiles[1] = rest[-1][3:]
+            ks.n_ops[1] += rest[-1][3]
+            ks.n_tiles[1] += rest[-1][4]
         fast = [(t, raw, tma) for c, t, raw, tma, _ in packed if c == 0]
         if fast:
             # stable split: TMA-capable ops first, relative order kept inside both groups
@@ -371,6 +380,8 @@ class CopyTable:
     def _launch_kernel(self, kernel, ops_ptr, tiles_ptr, n_ops, n_tiles, ctas_per_sm, sig, s) -> None:
         if kernel == "bulk":
             rc = self._lib.etha_m2n_bulk_launch(ops_ptr, tiles_ptr, n_ops, n_tiles, self._sync.data_ptr(), *sig, s)
+        elif isinstance(kernel, int) and kernel >= L.KEY_RAGGED:
+            rc = self._lib.etha_m2n_ragged_launch(ops_ptr, tiles_ptr, n_ops, kernel, n_tiles, self._sync.data_ptr(), *sig, s)
         elif isinstance(kernel, int):  # key of a streaming instance
             rc = self._lib.etha_m2n_typed_launch(ops_ptr, tiles_ptr, n_ops, kernel, n_tiles, self._sync.data_ptr(), *sig, s)
         else:
