@@ -232,6 +232,17 @@ __device__ __forceinline__ float reduce2(float a, float b, int op) {
   }
 }
 
+// a[k] = reduce2(a[k], b[k], op), with one branch on the op
+__device__ __forceinline__ void reduce8(float (&a)[8], const float (&b)[8], int op) {
+  if (op == M2N_SUM || op == M2N_AVG) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) a[k] += b[k];
+  } else {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) a[k] = reduce2(a[k], b[k], op);
+  }
+}
+
 template <int DT>
 __device__ __forceinline__ float round_through(float x) {
   if constexpr (DT == M2N_BF16) return __bfloat162float(__float2bfloat16_rn(x));

@@ -15,7 +15,8 @@ MAX_DIMS = 4
 DT_RAW, DT_F32, DT_BF16, DT_F16 = 0, 1, 2, 3
 RED_CODES = {"sum": 0, "avg": 1, "max": 2, "min": 3, "product": 4}
 FLAG_MULTIMEM = 1
-KEY_RAGGED = 0x1000  # keys from here on: ragged instances, below: streaming instances
+# instance keys: the kernel's name by `key >> 12`
+INSTANCE_KERNELS = {0: "typed", 1: "ragged", 2: "collapse"}
 STATUS_OK, STATUS_TIMEOUT, STATUS_BAD_OP = 0, 1, 2
 
 
@@ -82,10 +83,10 @@ def cuda_lib() -> C.CDLL:
         lib.etha_op_stream_key.restype = i32
         lib.etha_m2n_typed_launch.argtypes = [vp, vp, u32, i32, u32, vp, vp, u32, u32, i32, vp]
         lib.etha_m2n_typed_launch.restype = i32
-        lib.etha_op_ragged_key.argtypes = [vp]
-        lib.etha_op_ragged_key.restype = i32
-        lib.etha_m2n_ragged_launch.argtypes = [vp, vp, u32, i32, u32, vp, vp, u32, u32, i32, vp]
-        lib.etha_m2n_ragged_launch.restype = i32
+        for name in ("ragged", "collapse"):
+            key_of, launch = getattr(lib, f"etha_op_{name}_key"), getattr(lib, f"etha_m2n_{name}_launch")
+            key_of.argtypes, key_of.restype = [vp], i32
+            launch.argtypes, launch.restype = [vp, vp, u32, i32, u32, vp, vp, u32, u32, i32, vp], i32
         lib.etha_m2n_launch.argtypes = [vp, vp, u32, i32, u32, i32, vp, vp, u32, u32, i32, vp]
         lib.etha_m2n_launch.restype = i32
         lib.etha_set_flags.argtypes = [vp, u32, u32, vp]

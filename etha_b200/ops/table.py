@@ -189,7 +189,8 @@ class CopyTable:
                     tma = cls == 0 and bool(self._lib.etha_op_bulk_ok(buf))
                     skey = 0
                     if cls == 1 and self.stream_typed:
-                        skey = self._lib.etha_op_stream_key(buf) or self._lib.etha_op_ragged_key(buf)
+                        skey = (self._lib.etha_op_stream_key(buf) or self._lib.etha_op_collapse_key(buf)
+                                or self._lib.etha_op_ragged_key(buf))
                     entry = (cls, tiles, buf.raw, tma, skey)
                     self._packed.append(entry)
                     if dma_ok and self.dma_min_bytes is not None and numel * ddtype.itemsize >= self.dma_min_bytes:
@@ -232,14 +233,14 @@ class CopyTable:
 
         rest = []  # launches of the typed and general classes
         for key in dict.fromkeys(k for c, _, _, _, k in packed if c == 1 and k):
-            ragged = key >= L.KEY_RAGGED
-            rest.append(launch(key, [raw for c, _, raw, _, k in packed if c == 1 and k == key], 2 if ragged else 0))
-            if ragged:
-                ks.n_ops[1] += rest[-1][3]
-                ks.n_tiles[1] += rest[-1][4]
-            else:
+            kernel = L.INSTANCE_KERNELS[key >> 12]
+            rest.append(launch(key, [raw for c, _, raw, _, k in packed if c == 1 and k == key], 2 if kernel == "ragged" else 0))
+            if kernel == "typed":
                 ks.n_typed_ops += rest[-1][3]
                 ks.n_typed_tiles += rest[-1][4]
+            else:
+                ks.n_ops[1] += rest[-1][3]
+                ks.n_tiles[1] += rest[-1][4]
         general = [raw for c, _, raw, _, k in packed if c == 1 and not k]
         if general:
             rest.append(launch("general", general, 1))
@@ -380,10 +381,9 @@ class CopyTable:
     def _launch_kernel(self, kernel, ops_ptr, tiles_ptr, n_ops, n_tiles, ctas_per_sm, sig, s) -> None:
         if kernel == "bulk":
             rc = self._lib.etha_m2n_bulk_launch(ops_ptr, tiles_ptr, n_ops, n_tiles, self._sync.data_ptr(), *sig, s)
-        elif isinstance(kernel, int) and kernel >= L.KEY_RAGGED:
-            rc = self._lib.etha_m2n_ragged_launch(ops_ptr, tiles_ptr, n_ops, kernel, n_tiles, self._sync.data_ptr(), *sig, s)
-        elif isinstance(kernel, int):  # key of a streaming instance
-            rc = self._lib.etha_m2n_typed_launch(ops_ptr, tiles_ptr, n_ops, kernel, n_tiles, self._sync.data_ptr(), *sig, s)
+        elif isinstance(kernel, int):  # key of an instance
+            launch = getattr(self._lib, f"etha_m2n_{L.INSTANCE_KERNELS[kernel >> 12]}_launch")
+            rc = launch(ops_ptr, tiles_ptr, n_ops, kernel, n_tiles, self._sync.data_ptr(), *sig, s)
         else:
             rc = self._lib.etha_m2n_launch(ops_ptr, tiles_ptr, n_ops, int(kernel == "general"), n_tiles, ctas_per_sm,
                                            self._sync.data_ptr(), *sig, s)
