@@ -282,7 +282,7 @@ extern "C" {
 // M2N_KEY_RAGGED | (collapse << 8) | (source dtype << 4) | destination dtype (0 and 0: bit copy), or 0 when the op is not
 // of this class
 int etha_op_ragged_key(const M2NOp* op) {
-  if (!op->chunks) return 0;
+  if (!op->chunks || op->tr_flags) return 0;
   if (op->mode == M2N_MODE_RAW) return M2N_KEY_RAGGED;
   return M2N_KEY_RAGGED | ((op->mode == M2N_MODE_REDUCE) << 8) | (op->src_dtype << 4) | op->dst_dtype;
 }

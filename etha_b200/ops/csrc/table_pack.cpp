@@ -69,7 +69,16 @@ int64_t etha_layout_tiles(M2NOp* ops, uint32_t n_ops, int kernel, uint32_t* tile
   const uint32_t max_units = kernel == 1 ? 4096 : 1024, min_units = 256;
   const uint64_t ctas = 148 * 4;
   uint64_t total = 0, tiles = 0;
-  const auto count = [&](const M2NOp& op) { return kernel == 2 ? op.chunks : op.total_units; };
+  const auto count = [&](const M2NOp& op) { return kernel >= 2 ? op.chunks : op.total_units; };
+  if (kernel == 3) {  // a block of the transposing kernel is a tile
+    tile_start[0] = 0;
+    for (uint32_t i = 0; i < n_ops; ++i) {
+      ops[i].tile_units = 1;
+      if ((tiles += ops[i].chunks) >= (1ull << 31)) return -1;
+      tile_start[i + 1] = (uint32_t)tiles;
+    }
+    return (int64_t)tiles;
+  }
   for (uint32_t i = 0; i < n_ops; ++i) total += count(ops[i]);
   const uint64_t share = (total + ctas - 1) / ctas;
   const uint64_t units = std::min<uint64_t>(max_units, std::max<uint64_t>(min_units, (share + 255) / 256 * 256));
@@ -252,6 +261,35 @@ int etha_pack_op(const M2NOpSpec* s, M2NOp* o, char* err, int err_len) {
       o->chunks = (uint32_t)all;
       o->chunk_row = (uint32_t)per_row;
       magic((uint32_t)per_row, &o->chunk_mul, &o->chunk_shr);
+    }
+  }
+
+  // Transposing class: no dimension is contiguous on both sides, but one is on each.  Boxes narrower than 8 elements on
+  // either of the two leave most of a block empty and stay element-wise.
+  const bool elem = inner_elems == 1 && (mode == M2N_MODE_RAW ? (es == 2 || es == 4) && ubs == (uint32_t)es : mode == M2N_MODE_CVT);
+  if (elem && !(s->flags & M2N_FLAG_MULTIMEM) && aligned_all(es, ed)) {
+    int a = -1, b = -1;
+    for (size_t i = 0; i < dims.size(); ++i) {
+      if (dims[i].ds == 1 && a < 0) a = (int)i;
+      if (dims[i].ss == 1 && b < 0) b = (int)i;
+    }
+    if (a >= 0 && b >= 0 && a != b && dims[a].n >= 8 && dims[b].n >= 8) {
+      const int64_t kb = M2N_TRANSPOSE_B_BYTES / es;
+      int64_t blocks = (dims[a].n + M2N_TRANSPOSE_A - 1) / M2N_TRANSPOSE_A * ((dims[b].n + kb - 1) / kb);
+      bool src16 = true, dst16 = true;
+      for (int i = 0; i < s->nsrc; ++i) src16 = src16 && s->src[i] % 16 == 0;
+      for (int i = 0; i < s->ndst; ++i) dst16 = dst16 && s->dst[i] % 16 == 0;
+      for (size_t i = 0; i < dims.size(); ++i) {
+        if ((int)i != b) src16 = src16 && (dims[i].ss * es) % 16 == 0;
+        if ((int)i != a) dst16 = dst16 && (dims[i].ds * ed) % 16 == 0;
+        if ((int)i != a && (int)i != b) blocks *= dims[i].n;
+      }
+      if (blocks < (1ll << 31)) {
+        o->chunks = (uint32_t)blocks;
+        o->tr_flags = (uint8_t)(M2N_TR | (src16 ? M2N_TR_SRC16 : 0) | (dst16 ? M2N_TR_DST16 : 0));
+        o->tr_a = (uint8_t)a;
+        o->tr_b = (uint8_t)b;
+      }
     }
   }
   return 0;

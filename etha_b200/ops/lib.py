@@ -16,7 +16,7 @@ DT_RAW, DT_F32, DT_BF16, DT_F16 = 0, 1, 2, 3
 RED_CODES = {"sum": 0, "avg": 1, "max": 2, "min": 3, "product": 4}
 FLAG_MULTIMEM = 1
 # instance keys: the kernel's name by `key >> 12`
-INSTANCE_KERNELS = {0: "typed", 1: "ragged", 2: "collapse"}
+INSTANCE_KERNELS = {0: "typed", 1: "ragged", 2: "collapse", 3: "transpose"}
 STATUS_OK, STATUS_TIMEOUT, STATUS_BAD_OP = 0, 1, 2
 
 
@@ -83,7 +83,7 @@ def cuda_lib() -> C.CDLL:
         lib.etha_op_stream_key.restype = i32
         lib.etha_m2n_typed_launch.argtypes = [vp, vp, u32, i32, u32, vp, vp, u32, u32, i32, vp]
         lib.etha_m2n_typed_launch.restype = i32
-        for name in ("ragged", "collapse"):
+        for name in ("ragged", "collapse", "transpose"):
             key_of, launch = getattr(lib, f"etha_op_{name}_key"), getattr(lib, f"etha_m2n_{name}_launch")
             key_of.argtypes, key_of.restype = [vp], i32
             launch.argtypes, launch.restype = [vp, vp, u32, i32, u32, vp, vp, u32, u32, i32, vp], i32

@@ -190,7 +190,7 @@ class CopyTable:
                     skey = 0
                     if cls == 1 and self.stream_typed:
                         skey = (self._lib.etha_op_stream_key(buf) or self._lib.etha_op_collapse_key(buf)
-                                or self._lib.etha_op_ragged_key(buf))
+                                or self._lib.etha_op_ragged_key(buf) or self._lib.etha_op_transpose_key(buf))
                     entry = (cls, tiles, buf.raw, tma, skey)
                     self._packed.append(entry)
                     if dma_ok and self.dma_min_bytes is not None and numel * ddtype.itemsize >= self.dma_min_bytes:
@@ -234,7 +234,7 @@ class CopyTable:
         rest = []  # launches of the typed and general classes
         for key in dict.fromkeys(k for c, _, _, _, k in packed if c == 1 and k):
             kernel = L.INSTANCE_KERNELS[key >> 12]
-            rest.append(launch(key, [raw for c, _, raw, _, k in packed if c == 1 and k == key], 2 if kernel == "ragged" else 0))
+            rest.append(launch(key, [raw for c, _, raw, _, k in packed if c == 1 and k == key], {"ragged": 2, "transpose": 3}.get(kernel, 0)))
             if kernel == "typed":
                 ks.n_typed_ops += rest[-1][3]
                 ks.n_typed_tiles += rest[-1][4]
