@@ -2,11 +2,13 @@
 
 from __future__ import annotations
 
+from ctypes import byref as _byref
+
 import torch
 
 from . import lib as _L
 from .lib import STATUS_BAD_OP, STATUS_OK, STATUS_TIMEOUT, cuda_lib
-from .table import CopyTable, SliceRef, dtype_code
+from .table import LAUNCH_COUNT, CopyTable, SliceRef, dtype_code, make_spec, raw_stream
 
 FLAG_LAUNCH_COUNT = [0]  # set_flags / wait_flags kernels launched in this process
 
@@ -27,18 +29,27 @@ __all__ = [
 
 def local_copy(src: torch.Tensor, dst: torch.Tensor, stream: torch.cuda.Stream | None = None) -> None:
     """`dst[...] = src` (any strides, fp32/bf16/fp16 conversion) through the copy kernels."""
-    t = CopyTable(dst.device)
-    t.add_copy(src, dst)
-    t.finalize()
-    t.launch(stream)
-    # the table's device arrays must outlive the kernel: tie them to the stream
-    for buf in t.device_buffers():
-        buf.record_stream(stream or torch.cuda.current_stream(dst.device))
+    shape = tuple(src.shape)
+    if shape != tuple(dst.shape):
+        raise ValueError(f"shape mismatch {shape} vs {tuple(dst.shape)}")
+    if len(shape) > 8:
+        raise ValueError("at most 8 dims")
+    if not dst.is_cuda:
+        raise ValueError(f"the destination must be on a CUDA device, not on {dst.device}")
+    # one op, launched with the op in the kernel's arguments: no table is built or uploaded
+    spec = make_spec(shape, [SliceRef.of(src)], [SliceRef.of(dst)], (), (), 0, 0)
+    if not src.numel():
+        return
+    rc = cuda_lib().etha_run_spec(_byref(spec), raw_stream(stream, dst.device))
+    if -100 < rc < 0:  # refused by the packer
+        raise ValueError(f"cannot pack op ({rc}): {_L.last_error()}")
+    _L.check(rc, "local copy")
+    LAUNCH_COUNT[0] += 1
 
 
 def set_flags(addresses: torch.Tensor, epoch: int, stream: torch.cuda.Stream | None = None) -> None:
     """Store `epoch` (release, system scope) to every uint32 flag whose address is in `addresses` (int64, device)."""
-    s = (stream or torch.cuda.current_stream(addresses.device)).cuda_stream
+    s = raw_stream(stream, addresses.device)
     _L.check(cuda_lib().etha_set_flags(addresses.data_ptr(), addresses.numel(), epoch & 0xFFFFFFFF, s), "set_flags")
     FLAG_LAUNCH_COUNT[0] += 1
 
@@ -56,11 +67,10 @@ def wait_flags(
     `status` (int32[2], device or pinned-mapped) receives `[STATUS_OK | STATUS_TIMEOUT, index of the
     first missing flag]`.  The wait gives up after `timeout_s`; the context stays usable.
     """
-    s = (stream or torch.cuda.current_stream(flags.device)).cuda_stream
-    rc = cuda_lib().etha_wait_flags(
-        flags.data_ptr(), which.data_ptr(), which.numel(), epoch & 0xFFFFFFFF, int(timeout_s * 1e9), status.data_ptr(), s
-    )
-    _L.check(rc, "wait_flags")
+    rc = cuda_lib().etha_wait_flags(flags.data_ptr(), which.data_ptr(), which.numel(), epoch & 0xFFFFFFFF, int(timeout_s * 1e9),
+                                    status.data_ptr(), raw_stream(stream, flags.device))
+    if rc:
+        _L.check(rc, "wait_flags")
     FLAG_LAUNCH_COUNT[0] += 1
 
 

@@ -24,8 +24,8 @@
 #include <cstdio>
 
 #include "common.h"
-#include "m2n.h"
 #include "m2n_device.cuh"
+#include "m2n_launch.h"
 
 namespace {
 
@@ -140,8 +140,7 @@ __device__ __forceinline__ bool issue_fill(const M2NOp& op, uint32_t u0, uint32_
 }
 
 __global__ void __launch_bounds__(64, 1)
-m2n_bulk_kernel(const M2NOp* __restrict__ ops, const uint32_t* __restrict__ tile_start, uint32_t n_ops, uint32_t* sync,
-                const uint64_t* __restrict__ signals, uint32_t n_signals, uint32_t epoch, int do_signal) {
+m2n_bulk_kernel(const __grid_constant__ M2NLaunch args) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ uint32_t s_done;
   unsigned char* stage_buf = smem;  // kStages * kStageBytes
@@ -166,18 +165,9 @@ m2n_bulk_kernel(const M2NOp* __restrict__ ops, const uint32_t* __restrict__ tile
     while (alive) {
       if (lane == 0) sched_request(&ring.sched);
       if (tile < begin || tile >= end) {
-        uint32_t lo = 0, hi = n_ops;
-        while (hi - lo > 1) {
-          const uint32_t step = (hi - lo + 31) >> 5, i = lo + lane * step;
-          const uint32_t below = __ballot_sync(0xffffffffu, i < hi && tile_start[i] <= tile);
-          lo += (31 - __clz(below)) * step;
-          hi = min(hi, lo + step);
-        }
-        const uint4* g = reinterpret_cast<const uint4*>(ops + lo);
-        uint4* d = reinterpret_cast<uint4*>(&ring.op);
         __syncwarp();
-        for (uint32_t i = lane; i < sizeof(M2NOp) / 16; i += 32) d[i] = g[i];
-        begin = tile_start[lo], end = tile_start[lo + 1];
+        const uint2 tiles = load_op(args, tile, &ring.op);
+        begin = tiles.x, end = tiles.y;
         __syncwarp();
       }
       const M2NOp& op = ring.op;
@@ -185,18 +175,18 @@ m2n_bulk_kernel(const M2NOp* __restrict__ ops, const uint32_t* __restrict__ tile
       for (uint32_t u = first; u < limit && alive; u += kStageBytes / 16) {
         const uint32_t s = fills % kStages;
         if (!stage_free()) {
-          if (lane == 0) sync[1] = M2N_TIMEOUT;
+          if (lane == 0) report(args, M2N_TIMEOUT);
           alive = false;
         } else if (!issue_fill(op, u, min(limit, u + kStageBytes / 16), ring.meta[s], stage_buf + (size_t)s * kStageBytes,
                                &ring.full[s], lane)) {
-          if (lane == 0) sync[1] = M2N_BAD_OP;
+          if (lane == 0) report(args, M2N_BAD_OP);
           alive = false;
         } else {
           ++fills;
         }
       }
       ++done;
-      const bool more = sched_take(&ring.sched, phase, tile, sync);
+      const bool more = sched_take(&ring.sched, phase, tile, args);
       phase ^= 1;
       __syncwarp();
       alive = alive && more;
@@ -211,7 +201,7 @@ m2n_bulk_kernel(const M2NOp* __restrict__ ops, const uint32_t* __restrict__ tile
     for (uint32_t fill = 0;; ++fill) {
       const uint32_t s = fill % kStages;
       if (!mbar_wait(&ring.full[s], (fill / kStages) & 1)) {
-        if (lane == 0) sync[1] = M2N_TIMEOUT;
+        if (lane == 0) report(args, M2N_TIMEOUT);
         break;
       }
       const StageMeta& m = ring.meta[s];
@@ -231,17 +221,15 @@ m2n_bulk_kernel(const M2NOp* __restrict__ ops, const uint32_t* __restrict__ tile
     asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     asm volatile("fence.proxy.async;" ::: "memory");
   }
-  if (do_signal) {
+  if (args.do_signal) {
     __syncthreads();
-    finish_and_signal(sync, signals, n_signals, epoch, s_done, gridDim.x);
+    finish_and_signal(args, s_done);
   }
 }
 
 }  // namespace
 
-extern "C" int etha_m2n_bulk_launch(const M2NOp* ops, const uint32_t* tile_start, uint32_t n_ops, uint32_t n_tiles,
-                                    uint32_t* sync_scratch, const uint64_t* signals, uint32_t n_signals, uint32_t epoch,
-                                    int do_signal, void* stream) {
+int m2n_launch_bulk(const M2NLaunch& args, uint32_t n_tiles, void* stream) {
   static bool configured[64] = {false};
   const size_t smem = (size_t)kStages * kStageBytes + sizeof(Ring);
   int dev = 0;
@@ -254,13 +242,5 @@ extern "C" int etha_m2n_bulk_launch(const M2NOp* ops, const uint32_t* tile_start
     }
     configured[dev] = true;
   }
-  if (!n_tiles) return 0;
-  m2n_bulk_kernel<<<n_tiles, 64, smem, (cudaStream_t)stream>>>(ops, tile_start, n_ops, sync_scratch, signals, n_signals, epoch,
-                                                            do_signal);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) {
-    snprintf(etha_err_buf(), ETHA_ERR_LEN, "bulk kernel launch: %s", cudaGetErrorString(e));
-    return -(int)e - 1000;
-  }
-  return 0;
+  return m2n_launch(m2n_bulk_kernel, n_tiles, 64, smem, stream, args, "bulk");
 }

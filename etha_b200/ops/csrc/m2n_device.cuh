@@ -10,6 +10,7 @@
 #include <type_traits>
 
 #include "m2n.h"
+#include "m2n_launch.h"
 
 namespace {
 
@@ -261,17 +262,21 @@ __device__ __forceinline__ float round_through(float x) {
 // and four writes: 5.6 and 6.6.  Why not a counter in memory: the hardware's queue belongs to the launch, so two launches of one table (two
 // streams, a graph) share nothing and nothing has to be reset.  A CTA that takes tiles over pays its prologue (and the
 // completion fence) once.
+__device__ __forceinline__ void report(const M2NLaunch& args, uint32_t status) {
+  if (args.sync) args.sync[1] = status;
+}
+
 struct TileSched {
   uint4 handle;  // answer of try_cancel, written by the asynchronous proxy
   uint64_t bar;
-  uint32_t op, begin, end;  // op in `s_op` and its tiles [begin, end)
+  uint32_t begin, end;  // tiles of the op in `s_op`
 };
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void sched_init(TileSched* s) {
   if (threadIdx.x == 0) {
-    s->op = 0xffffffffu, s->begin = 1, s->end = 0;
+    s->begin = 1, s->end = 0;
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&s->bar)));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -291,7 +296,7 @@ __device__ __forceinline__ void sched_request(TileSched* s) {
 
 // every thread waits (bounded) for the answer; returns false when no tile is left.  The caller synchronises the CTA
 // before the next request.
-__device__ __forceinline__ bool sched_take(TileSched* s, uint32_t phase, uint32_t& tile, uint32_t* sync) {
+__device__ __forceinline__ bool sched_take(TileSched* s, uint32_t phase, uint32_t& tile, const M2NLaunch& args) {
   const uint32_t bar = smem_addr(&s->bar);
   uint32_t ready = 0;
   for (uint32_t spin = 0; spin < (1u << 22) && !ready; ++spin) {
@@ -304,7 +309,7 @@ __device__ __forceinline__ bool sched_take(TileSched* s, uint32_t phase, uint32_
         : "memory");
   }
   if (!ready) {
-    sync[1] = M2N_TIMEOUT;
+    report(args, M2N_TIMEOUT);
     return false;
   }
   uint32_t more;
@@ -322,26 +327,36 @@ __device__ __forceinline__ bool sched_take(TileSched* s, uint32_t phase, uint32_
   return more != 0;
 }
 
-// (re)load the op that owns `tile` into shared memory; the CTA is synchronised since the last use of `s_op`.  Tiles come
-// in ascending order, so the op is nearly always the one already there; otherwise warp 0 looks it up 32 ways at a time.
-__device__ __forceinline__ void sched_locate(TileSched* s, const M2NOp* __restrict__ ops,
-                                             const uint32_t* __restrict__ tile_start, uint32_t n_ops, uint32_t tile,
-                                             M2NOp* s_op) {
-  if (tile >= s->begin && tile < s->end) return;
-  __syncthreads();  // everybody has read begin / end
-  if (threadIdx.x < 32) {
-    const uint32_t lane = threadIdx.x;
-    uint32_t lo = 0, hi = n_ops;
+// one warp loads the op that owns `tile` (looked up 32 ways at a time) into shared memory; returns its tiles
+__device__ __forceinline__ uint2 load_op(const M2NLaunch& args, uint32_t tile, M2NOp* s_op) {
+  const uint32_t lane = threadIdx.x & 31;
+  const M2NOp* op = &args.one;
+  uint2 tiles = make_uint2(0, gridDim.x);
+  if (args.ops) {
+    uint32_t lo = 0, hi = args.n_ops;
     while (hi - lo > 1) {
       const uint32_t step = (hi - lo + 31) >> 5, i = lo + lane * step;
-      const uint32_t below = __ballot_sync(0xffffffffu, i < hi && tile_start[i] <= tile);
+      const uint32_t below = __ballot_sync(0xffffffffu, i < hi && args.tile_start[i] <= tile);
       lo += (31 - __clz(below)) * step;
       hi = min(hi, lo + step);
     }
-    const uint4* g = reinterpret_cast<const uint4*>(ops + lo);
-    uint4* d = reinterpret_cast<uint4*>(s_op);
-    for (uint32_t i = lane; i < sizeof(M2NOp) / 16; i += 32) d[i] = g[i];
-    if (lane == 0) s->op = lo, s->begin = tile_start[lo], s->end = tile_start[lo + 1];
+    op = args.ops + lo;
+    tiles = make_uint2(args.tile_start[lo], args.tile_start[lo + 1]);
+  }
+  const uint4* g = reinterpret_cast<const uint4*>(op);
+  uint4* d = reinterpret_cast<uint4*>(s_op);
+  for (uint32_t i = lane; i < sizeof(M2NOp) / 16; i += 32) d[i] = g[i];
+  return tiles;
+}
+
+// make `s_op` the op that owns `tile`; the CTA is synchronised since its last use.  Tiles come in ascending order, so the
+// op is nearly always the one already there.
+__device__ __forceinline__ void sched_locate(TileSched* s, const M2NLaunch& args, uint32_t tile, M2NOp* s_op) {
+  if (tile >= s->begin && tile < s->end) return;
+  __syncthreads();  // everybody has read begin / end
+  if (threadIdx.x < 32) {
+    const uint2 tiles = load_op(args, tile, s_op);
+    if (threadIdx.x == 0) s->begin = tiles.x, s->end = tiles.y;
   }
   __syncthreads();
 }
@@ -349,19 +364,17 @@ __device__ __forceinline__ void sched_locate(TileSched* s, const M2NOp* __restri
 // Walk over all tiles of the table: `body(op, first unit, one past the last unit)` runs with all threads of the CTA.
 // Returns the number of tiles this CTA ran.  CHUNKS: the tiles are counted in the op's chunks instead of its units.
 template <bool CHUNKS = false, typename Body>
-__device__ __forceinline__ uint32_t for_each_tile(TileSched* s, M2NOp* s_op, const M2NOp* __restrict__ ops,
-                                                  const uint32_t* __restrict__ tile_start, uint32_t n_ops, uint32_t* sync,
-                                                  Body&& body) {
+__device__ __forceinline__ uint32_t for_each_tile(TileSched* s, M2NOp* s_op, const M2NLaunch& args, Body&& body) {
   sched_init(s);
   uint32_t tile = blockIdx.x, done = 0, phase = 0;
   while (true) {
     if (threadIdx.x == 0) sched_request(s);
-    sched_locate(s, ops, tile_start, n_ops, tile, s_op);
+    sched_locate(s, args, tile, s_op);
     const M2NOp& op = *s_op;
     const uint32_t base = (tile - s->begin) * op.tile_units;
     body(op, base, min(CHUNKS ? op.chunks : op.total_units, base + op.tile_units));
     ++done;
-    const bool more = sched_take(s, phase, tile, sync);
+    const bool more = sched_take(s, phase, tile, args);
     phase ^= 1;
     __syncthreads();
     if (!more) return done;
@@ -373,22 +386,21 @@ __device__ __forceinline__ uint32_t for_each_tile(TileSched* s, M2NOp* s_op, con
 // its system-scope release stores order them for the consumers too (release patterns are cumulative).  What a small table
 // of 592 CTAs pays for its signal: 13 us with a system-scope fence in every CTA, 5 us with a GPU-scope one there and a
 // system-scope fence before the release stores, 3 us as it stands.
-__device__ __forceinline__ void finish_and_signal(uint32_t* sync, const uint64_t* signals, uint32_t n_signals,
-                                                  uint32_t epoch, uint32_t done, uint32_t total) {
+__device__ __forceinline__ void finish_and_signal(const M2NLaunch& args, uint32_t done) {
   __shared__ uint32_t s_last;
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
-    const uint32_t prev = atomicAdd(&sync[0], done);
-    s_last = (prev + done == total) ? 1u : 0u;
+    const uint32_t prev = atomicAdd(&args.sync[0], done);
+    s_last = (prev + done == gridDim.x) ? 1u : 0u;
     __threadfence();
   }
   __syncthreads();
   if (s_last) {
-    if (threadIdx.x == 0) sync[0] = 0;  // ready for the next launch on this stream
-    for (uint32_t i = threadIdx.x; i < n_signals; i += blockDim.x) {
-      uint32_t* flag = reinterpret_cast<uint32_t*>(signals[i]);
-      asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(flag), "r"(epoch) : "memory");
+    if (threadIdx.x == 0) args.sync[0] = 0;  // ready for the next launch on this stream
+    for (uint32_t i = threadIdx.x; i < args.n_signals; i += blockDim.x) {
+      uint32_t* flag = reinterpret_cast<uint32_t*>(args.signals[i]);
+      asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(flag), "r"(args.epoch) : "memory");
     }
   }
 }

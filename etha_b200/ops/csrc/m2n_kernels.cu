@@ -7,8 +7,6 @@
 // consumers' slices over NVLink.  This replaces the reference's per-chunk slice/contiguous/cast/
 // pack kernels and its NCCL send/recv/broadcast/all-reduce calls (src/etha/comm/ir.py:101-141,
 // 229-310; src/etha/comm/transfer.py:20-41).
-#include "m2n.h"
-
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -18,6 +16,7 @@
 
 #include "common.h"
 #include "m2n_device.cuh"
+#include "m2n_launch.h"
 
 namespace {
 
@@ -299,16 +298,14 @@ __device__ __forceinline__ void fast_tile(const M2NOp& op, uint32_t base, uint32
 }
 
 __global__ void __launch_bounds__(kFastThreads, kFastCtas)
-m2n_fast_kernel(const M2NOp* __restrict__ ops, const uint32_t* __restrict__ tile_start, uint32_t n_ops, uint32_t* sync,
-                const uint64_t* __restrict__ signals, uint32_t n_signals, uint32_t epoch, int do_signal) {
+m2n_fast_kernel(const __grid_constant__ M2NLaunch args) {
   __shared__ M2NOp s_op;
   __shared__ TileSched s_sched;
-  const uint32_t done = for_each_tile(&s_sched, &s_op, ops, tile_start, n_ops, sync,
-                                      [](const M2NOp& op, uint32_t base, uint32_t limit) {
+  const uint32_t done = for_each_tile(&s_sched, &s_op, args, [&](const M2NOp& op, uint32_t base, uint32_t limit) {
     if (op.ndim == 0) fast_tile<0>(op, base, limit);
     else fast_tile<1>(op, base, limit);
   });
-  if (do_signal) finish_and_signal(sync, signals, n_signals, epoch, done, gridDim.x);
+  if (args.do_signal) finish_and_signal(args, done);
 }
 
 // General class: any other bit copy, converting copies and Partial collapses.
@@ -320,13 +317,10 @@ __device__ __noinline__ void walk_raw(const M2NOp& op, uint32_t base, uint32_t l
 }
 
 __global__ void __launch_bounds__(kGeneralThreads, ETHA_GENERAL_CTAS)
-m2n_general_kernel(const M2NOp* __restrict__ ops, const uint32_t* __restrict__ tile_start, uint32_t n_ops,
-                   uint32_t* sync, const uint64_t* __restrict__ signals, uint32_t n_signals, uint32_t epoch,
-                   int do_signal) {
+m2n_general_kernel(const __grid_constant__ M2NLaunch args) {
   __shared__ M2NOp s_op;
   __shared__ TileSched s_sched;
-  const uint32_t done = for_each_tile(&s_sched, &s_op, ops, tile_start, n_ops, sync,
-                                      [sync](const M2NOp& op, uint32_t base, uint32_t limit) {
+  const uint32_t done = for_each_tile(&s_sched, &s_op, args, [&](const M2NOp& op, uint32_t base, uint32_t limit) {
     if (op.mode == M2N_MODE_RAW) {
       switch (op.unit_bytes_src) {
         case 16: walk_raw<uint4>(op, base, limit); break;
@@ -336,10 +330,10 @@ m2n_general_kernel(const M2NOp* __restrict__ ops, const uint32_t* __restrict__ t
         default: walk_raw<uint8_t>(op, base, limit); break;
       }
     } else if (!dispatch_typed(op, base, limit)) {
-      if (threadIdx.x == 0) sync[1] = M2N_BAD_OP;
+      if (threadIdx.x == 0) report(args, M2N_BAD_OP);
     }
   });
-  if (do_signal) finish_and_signal(sync, signals, n_signals, epoch, done, gridDim.x);
+  if (args.do_signal) finish_and_signal(args, done);
 }
 
 __global__ void set_flags_kernel(const uint64_t* __restrict__ signals, uint32_t n_signals, uint32_t epoch) {
@@ -390,30 +384,19 @@ inline int fail(cudaError_t e, const char* what) {
 
 }  // namespace
 
-extern "C" {
-
-int etha_m2n_launch(const M2NOp* ops, const uint32_t* tile_start, uint32_t n_ops, int general, uint32_t n_tiles,
-                    int ctas_per_sm, uint32_t* sync_scratch, const uint64_t* signals, uint32_t n_signals, uint32_t epoch,
-                    int do_signal, void* stream) {
-  if (!n_tiles) return 0;
-  cudaStream_t s = (cudaStream_t)stream;
-  if (general) {
-    m2n_general_kernel<<<n_tiles, kGeneralThreads, 0, s>>>(ops, tile_start, n_ops, sync_scratch, signals, n_signals, epoch,
-                                                           do_signal);
-  } else {
-    // a caller that asks for one CTA per SM (of the two that fill it by default) leaves half of each SM to other work:
-    // shared memory that is never touched lets two of the four CTAs in
-    const int smem = ctas_per_sm == 1 ? 76 * 1024 : 0;
-    if (smem) {
-      cudaError_t e = cudaFuncSetAttribute(m2n_fast_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-      if (e != cudaSuccess) return fail(e, "fast kernel shared memory opt-in");
-    }
-    m2n_fast_kernel<<<n_tiles, kFastThreads, smem, s>>>(ops, tile_start, n_ops, sync_scratch, signals, n_signals, epoch,
-                                                        do_signal);
+int m2n_launch_copy(const M2NLaunch& args, bool general, uint32_t n_tiles, int ctas_per_sm, void* stream) {
+  if (general) return m2n_launch(m2n_general_kernel, n_tiles, kGeneralThreads, 0, stream, args, "general");
+  // a caller that asks for one CTA per SM (of the two that fill it by default) leaves half of each SM to other work:
+  // shared memory that is never touched lets two of the four CTAs in
+  const int smem = ctas_per_sm == 1 ? 76 * 1024 : 0;
+  if (smem) {
+    cudaError_t e = cudaFuncSetAttribute(m2n_fast_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return fail(e, "fast kernel shared memory opt-in");
   }
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : fail(e, "m2n kernel launch");
+  return m2n_launch(m2n_fast_kernel, n_tiles, kFastThreads, smem, stream, args, "fast");
 }
+
+extern "C" {
 
 int etha_set_flags(const uint64_t* signals, uint32_t n_signals, uint32_t epoch, void* stream) {
   set_flags_kernel<<<1, 64, 0, (cudaStream_t)stream>>>(signals, n_signals, epoch);
@@ -472,11 +455,6 @@ int noalloc_setup(int dev, unsigned char** out) {
 
 }  // namespace
 
-extern "C" int etha_pack_op(const M2NOpSpec* spec, M2NOp* out, char* err, int err_len);
-extern "C" uint32_t etha_op_tiles(const M2NOp* op);
-extern "C" int etha_op_class(const M2NOp* op);
-extern "C" int64_t etha_layout_tiles(M2NOp* ops, uint32_t n_ops, int kernel, uint32_t* tile_start);
-
 extern "C" int etha_m2n_run_noalloc(const M2NOpSpec* specs, uint32_t n_specs, int ctas_per_sm, void* stream) {
   if (!specs && n_specs) {
     snprintf(etha_err_buf(), ETHA_ERR_LEN, "null spec array");
@@ -534,8 +512,9 @@ extern "C" int etha_m2n_run_noalloc(const M2NOpSpec* specs, uint32_t n_specs, in
     if (e != cudaSuccess) return fail(e, "cudaMemcpyAsync(tile table)");
     e = cudaMemcpyAsync(class_ops, packed[c], count[c] * sizeof(M2NOp), cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) return fail(e, "cudaMemcpyAsync(op table)");
-    uint32_t* sync = reinterpret_cast<uint32_t*>(scratch + 256 * c);
-    rc = etha_m2n_launch(class_ops, tiles_dev, count[c], c, tile_start[c][count[c]], ctas_per_sm, sync, nullptr, 0, 0, 0, s);
+    const EthaLaunch launch = {c == 0 ? M2N_KEY_FAST : M2N_KEY_GENERAL, count[c], tile_start[c][count[c]], 0,
+                               reinterpret_cast<uint64_t>(class_ops), reinterpret_cast<uint64_t>(tiles_dev)};
+    rc = etha_run(&launch, 1, reinterpret_cast<uint32_t*>(scratch + 256 * c), nullptr, 0, 0, ctas_per_sm, s);
     if (rc != 0) return rc;
   }
   return 0;

@@ -1,0 +1,43 @@
+// What the kernels of the copy table take, and the launchers of the kernel families (internal to the library).
+#pragma once
+#include <cuda_runtime.h>
+
+#include <cstdio>
+
+#include "common.h"
+#include "m2n.h"
+
+// The one argument of every kernel, in the constant bank.  A launch of a single op can carry it here (`ops` null): nothing
+// has to be uploaded and the op is not fetched from memory.
+struct M2NLaunch {
+  const M2NOp* ops;
+  const uint32_t* tile_start;
+  uint32_t n_ops;
+  uint32_t* sync;  // finished tiles, error word; may be null where nothing is signalled
+  const uint64_t* signals;
+  uint32_t n_signals;
+  uint32_t epoch;
+  int do_signal;
+  M2NOp one;
+};
+
+template <typename Kernel>
+inline int m2n_launch(Kernel kernel, uint32_t grid, int block, size_t smem, void* stream, const M2NLaunch& args, const char* what) {
+  kernel<<<grid, block, smem, (cudaStream_t)stream>>>(args);
+  const cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) return 0;
+  snprintf(etha_err_buf(), ETHA_ERR_LEN, "%s kernel launch: %s", what, cudaGetErrorString(e));
+  return -(int)e - 1000;
+}
+
+inline int m2n_no_instance(const char* what, int key) {
+  snprintf(etha_err_buf(), ETHA_ERR_LEN, "no %s kernel instance for key 0x%x", what, key);
+  return -102;
+}
+
+int m2n_launch_copy(const M2NLaunch& args, bool general, uint32_t n_tiles, int ctas_per_sm, void* stream);
+int m2n_launch_bulk(const M2NLaunch& args, uint32_t n_tiles, void* stream);
+int m2n_launch_typed(const M2NLaunch& args, int key, uint32_t n_tiles, void* stream);
+int m2n_launch_collapse(const M2NLaunch& args, int key, uint32_t n_tiles, void* stream);
+int m2n_launch_ragged(const M2NLaunch& args, int key, uint32_t n_tiles, void* stream);
+int m2n_launch_transpose(const M2NLaunch& args, int key, uint32_t n_tiles, void* stream);

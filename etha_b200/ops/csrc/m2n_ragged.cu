@@ -16,8 +16,8 @@
 #include <type_traits>
 
 #include "common.h"
-#include "m2n.h"
 #include "m2n_device.cuh"
+#include "m2n_launch.h"
 
 namespace {
 
@@ -249,17 +249,15 @@ __device__ __forceinline__ void typed_trip(const M2NOp& op, uint32_t chunk0) {
 
 template <int SDT, int DDT, bool REDUCE>
 __global__ void __launch_bounds__(kRaggedThreads, kRaggedCtas<SDT, REDUCE>)
-m2n_ragged_kernel(const M2NOp* __restrict__ ops, const uint32_t* __restrict__ tile_start, uint32_t n_ops, uint32_t* sync,
-                  const uint64_t* __restrict__ signals, uint32_t n_signals, uint32_t epoch, int do_signal) {
+m2n_ragged_kernel(const __grid_constant__ M2NLaunch args) {
   __shared__ M2NOp s_op;
   __shared__ TileSched s_sched;
   constexpr int U = kRaggedUnroll;
   constexpr int kMode = SDT == M2N_RAW ? M2N_MODE_RAW : (REDUCE ? M2N_MODE_REDUCE : M2N_MODE_CVT);
-  const uint32_t done = for_each_tile<true>(&s_sched, &s_op, ops, tile_start, n_ops, sync,
-                                            [sync](const M2NOp& op, uint32_t base, uint32_t limit) {
+  const uint32_t done = for_each_tile<true>(&s_sched, &s_op, args, [&](const M2NOp& op, uint32_t base, uint32_t limit) {
     // the host only puts ops of this instance into the table; anything else is reported, not executed
     if (!op.chunks || op.mode != kMode || (SDT != M2N_RAW && (op.src_dtype != SDT || op.dst_dtype != DDT))) {
-      if (threadIdx.x == 0) sync[1] = M2N_BAD_OP;
+      if (threadIdx.x == 0) report(args, M2N_BAD_OP);
       return;
     }
     const auto trip = [&](auto units, uint32_t chunk0) {
@@ -272,7 +270,7 @@ m2n_ragged_kernel(const M2NOp* __restrict__ ops, const uint32_t* __restrict__ ti
 #pragma unroll 1
     for (b += threadIdx.x; b < limit; b += kRaggedThreads) trip(std::integral_constant<int, 1>(), b);
   });
-  if (do_signal) finish_and_signal(sync, signals, n_signals, epoch, done, gridDim.x);
+  if (args.do_signal) finish_and_signal(args, done);
 }
 
 }  // namespace
@@ -287,16 +285,11 @@ int etha_op_ragged_key(const M2NOp* op) {
   return M2N_KEY_RAGGED | ((op->mode == M2N_MODE_REDUCE) << 8) | (op->src_dtype << 4) | op->dst_dtype;
 }
 
-int etha_m2n_ragged_launch(const M2NOp* ops, const uint32_t* tile_start, uint32_t n_ops, int key, uint32_t n_tiles,
-                           uint32_t* sync_scratch, const uint64_t* signals, uint32_t n_signals, uint32_t epoch, int do_signal,
-                           void* stream) {
-  if (!n_tiles) return 0;
-  cudaStream_t st = (cudaStream_t)stream;
-#define CASE(S, D, R)                                                                                                    \
-  case (R << 8) | (S << 4) | D:                                                                                          \
-    m2n_ragged_kernel<S, D, R><<<n_tiles, kRaggedThreads, 0, st>>>(ops, tile_start, n_ops, sync_scratch, signals, n_signals, \
-                                                                epoch, do_signal);                                       \
-    break;
+}  // extern "C"
+
+int m2n_launch_ragged(const M2NLaunch& args, int key, uint32_t n_tiles, void* stream) {
+#define CASE(S, D, R) \
+  case (R << 8) | (S << 4) | D: return m2n_launch(m2n_ragged_kernel<S, D, R>, n_tiles, kRaggedThreads, 0, stream, args, "ragged");
   switch (key & 0x1ff) {
     CASE(M2N_RAW, M2N_RAW, 0)
     CASE(M2N_F32, M2N_BF16, 0) CASE(M2N_F32, M2N_F16, 0) CASE(M2N_BF16, M2N_F32, 0)
@@ -304,17 +297,7 @@ int etha_m2n_ragged_launch(const M2NOp* ops, const uint32_t* tile_start, uint32_
     CASE(M2N_F32, M2N_F32, 1) CASE(M2N_F32, M2N_BF16, 1) CASE(M2N_F32, M2N_F16, 1)
     CASE(M2N_BF16, M2N_F32, 1) CASE(M2N_BF16, M2N_BF16, 1) CASE(M2N_BF16, M2N_F16, 1)
     CASE(M2N_F16, M2N_F32, 1) CASE(M2N_F16, M2N_BF16, 1) CASE(M2N_F16, M2N_F16, 1)
-    default:
-      snprintf(etha_err_buf(), ETHA_ERR_LEN, "no ragged kernel instance for key 0x%x", key);
-      return -102;
+    default: return m2n_no_instance("ragged", key);
   }
 #undef CASE
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) {
-    snprintf(etha_err_buf(), ETHA_ERR_LEN, "ragged kernel launch: %s", cudaGetErrorString(e));
-    return -(int)e - 1000;
-  }
-  return 0;
 }
-
-}  // extern "C"

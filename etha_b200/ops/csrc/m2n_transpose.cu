@@ -17,8 +17,8 @@
 #include <cstdio>
 
 #include "common.h"
-#include "m2n.h"
 #include "m2n_device.cuh"
+#include "m2n_launch.h"
 
 namespace {
 
@@ -185,22 +185,20 @@ __device__ __forceinline__ void block_move(const M2NOp& op, uint32_t block, uint
 
 template <int SDT, int DDT, int ES>
 __global__ void __launch_bounds__(kThreads, 5)
-m2n_transpose_kernel(const M2NOp* __restrict__ ops, const uint32_t* __restrict__ tile_start, uint32_t n_ops, uint32_t* sync,
-                     const uint64_t* __restrict__ signals, uint32_t n_signals, uint32_t epoch, int do_signal) {
+m2n_transpose_kernel(const __grid_constant__ M2NLaunch args) {
   __shared__ M2NOp s_op;
   __shared__ TileSched s_sched;
   __shared__ __align__(16) uint32_t s_tile[kA * kRowWords];
-  const uint32_t done = for_each_tile<true>(&s_sched, &s_op, ops, tile_start, n_ops, sync,
-                                            [sync](const M2NOp& op, uint32_t base, uint32_t limit) {
+  const uint32_t done = for_each_tile<true>(&s_sched, &s_op, args, [&](const M2NOp& op, uint32_t base, uint32_t limit) {
     // the host only puts ops of this instance into the table; anything else is reported, not executed
     if (!(op.tr_flags & M2N_TR) || (SDT == M2N_RAW ? (op.mode != M2N_MODE_RAW || op.unit_bytes_src != ES)
                                                    : (op.src_dtype != SDT || op.dst_dtype != DDT))) {
-      if (threadIdx.x == 0) sync[1] = M2N_BAD_OP;
+      if (threadIdx.x == 0) report(args, M2N_BAD_OP);
       return;
     }
     for (uint32_t b = base; b < limit; ++b) block_move<SDT, DDT, ES>(op, b, s_tile);
   });
-  if (do_signal) finish_and_signal(sync, signals, n_signals, epoch, done, gridDim.x);
+  if (args.do_signal) finish_and_signal(args, done);
 }
 
 }  // namespace
@@ -214,33 +212,18 @@ int etha_op_transpose_key(const M2NOp* op) {
   return M2N_KEY_TRANSPOSE | (op->src_dtype << 4) | op->dst_dtype;
 }
 
-int etha_m2n_transpose_launch(const M2NOp* ops, const uint32_t* tile_start, uint32_t n_ops, int key, uint32_t n_tiles,
-                              uint32_t* sync_scratch, const uint64_t* signals, uint32_t n_signals, uint32_t epoch,
-                              int do_signal, void* stream) {
-  if (!n_tiles) return 0;
-  cudaStream_t st = (cudaStream_t)stream;
-#define CASE(KEY, S, D, ES)                                                                                            \
-  case KEY:                                                                                                            \
-    m2n_transpose_kernel<S, D, ES><<<n_tiles, kThreads, 0, st>>>(ops, tile_start, n_ops, sync_scratch, signals, n_signals, \
-                                                                 epoch, do_signal);                                    \
-    break;
+}  // extern "C"
+
+int m2n_launch_transpose(const M2NLaunch& args, int key, uint32_t n_tiles, void* stream) {
+#define CASE(KEY, S, D, ES) \
+  case KEY: return m2n_launch(m2n_transpose_kernel<S, D, ES>, n_tiles, kThreads, 0, stream, args, "transposing");
 #define CVT(S, D, ES) CASE((S << 4) | D, S, D, ES)
   switch (key & 0xfff) {
     CASE(2 << 8, M2N_RAW, M2N_RAW, 2) CASE(4 << 8, M2N_RAW, M2N_RAW, 4)
     CVT(M2N_F32, M2N_BF16, 4) CVT(M2N_F32, M2N_F16, 4) CVT(M2N_BF16, M2N_F32, 2)
     CVT(M2N_BF16, M2N_F16, 2) CVT(M2N_F16, M2N_F32, 2) CVT(M2N_F16, M2N_BF16, 2)
-    default:
-      snprintf(etha_err_buf(), ETHA_ERR_LEN, "no transposing kernel instance for key 0x%x", key);
-      return -102;
+    default: return m2n_no_instance("transposing", key);
   }
 #undef CVT
 #undef CASE
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) {
-    snprintf(etha_err_buf(), ETHA_ERR_LEN, "transposing kernel launch: %s", cudaGetErrorString(e));
-    return -(int)e - 1000;
-  }
-  return 0;
 }
-
-}  // extern "C"

@@ -18,8 +18,8 @@
 #include <cstdio>
 
 #include "common.h"
-#include "m2n.h"
 #include "m2n_device.cuh"
+#include "m2n_launch.h"
 
 namespace {
 
@@ -92,21 +92,19 @@ __device__ __forceinline__ void stream_tile(const M2NOp& op, uint32_t base, uint
 
 template <int SDT, int DDT, int NSRC>
 __global__ void __launch_bounds__(kTypedThreads, kTypedCtasPerSm)
-m2n_typed_kernel(const M2NOp* __restrict__ ops, const uint32_t* __restrict__ tile_start, uint32_t n_ops, uint32_t* sync,
-                 const uint64_t* __restrict__ signals, uint32_t n_signals, uint32_t epoch, int do_signal) {
+m2n_typed_kernel(const __grid_constant__ M2NLaunch args) {
   __shared__ M2NOp s_op;
   __shared__ TileSched s_sched;
-  const uint32_t done = for_each_tile(&s_sched, &s_op, ops, tile_start, n_ops, sync,
-                                      [sync](const M2NOp& op, uint32_t base, uint32_t limit) {
+  const uint32_t done = for_each_tile(&s_sched, &s_op, args, [&](const M2NOp& op, uint32_t base, uint32_t limit) {
     // the host only puts ops of this instance's key into the table; anything else is reported, not executed
     if (op.src_dtype != SDT || op.dst_dtype != DDT || op.nsrc != NSRC || op.unit_elems != 8 || op.ndim > 1) {
-      if (threadIdx.x == 0) sync[1] = M2N_BAD_OP;
+      if (threadIdx.x == 0) report(args, M2N_BAD_OP);
       return;
     }
     if (op.ndim == 0) stream_tile<SDT, DDT, NSRC, 0>(op, base, limit);
     else stream_tile<SDT, DDT, NSRC, 1>(op, base, limit);
   });
-  if (do_signal) finish_and_signal(sync, signals, n_signals, epoch, done, gridDim.x);
+  if (args.do_signal) finish_and_signal(args, done);
 }
 
 // Collapses without an instance of their own (3 or 5 to 8 sources, two levels, the two 16-bit types mixed): one kernel per
@@ -196,15 +194,13 @@ __device__ __forceinline__ void collapse_trip(const M2NOp& op, uint32_t unit0) {
 
 template <int SDT, int DDT, bool TWO>
 __global__ void __launch_bounds__(kTypedThreads, kTypedCtasPerSm)
-m2n_collapse_kernel(const M2NOp* __restrict__ ops, const uint32_t* __restrict__ tile_start, uint32_t n_ops, uint32_t* sync,
-                    const uint64_t* __restrict__ signals, uint32_t n_signals, uint32_t epoch, int do_signal) {
+m2n_collapse_kernel(const __grid_constant__ M2NLaunch args) {
   __shared__ M2NOp s_op;
   __shared__ TileSched s_sched;
-  const uint32_t done = for_each_tile(&s_sched, &s_op, ops, tile_start, n_ops, sync,
-                                      [sync](const M2NOp& op, uint32_t base, uint32_t limit) {
+  const uint32_t done = for_each_tile(&s_sched, &s_op, args, [&](const M2NOp& op, uint32_t base, uint32_t limit) {
     if (op.mode != M2N_MODE_REDUCE || op.src_dtype != SDT || op.dst_dtype != DDT || op.unit_elems != 8 || op.ndim > 1 ||
         (op.red_size[1] > 1) != TWO) {
-      if (threadIdx.x == 0) sync[1] = M2N_BAD_OP;
+      if (threadIdx.x == 0) report(args, M2N_BAD_OP);
       return;
     }
     // a single run is a matrix of one row: its row index and its strides are 0
@@ -215,7 +211,7 @@ m2n_collapse_kernel(const M2NOp* __restrict__ ops, const uint32_t* __restrict__ 
 #pragma unroll 1
     for (b += threadIdx.x; b < limit; b += kTypedThreads) collapse_trip<SDT, DDT, TWO, 1>(op, b);
   });
-  if (do_signal) finish_and_signal(sync, signals, n_signals, epoch, done, gridDim.x);
+  if (args.do_signal) finish_and_signal(args, done);
 }
 
 constexpr bool typed(int dt) { return dt == M2N_F32 || dt == M2N_BF16 || dt == M2N_F16; }
@@ -230,36 +226,9 @@ constexpr bool has_instance(int s, int d, int n) {
 }
 
 template <int S, int D, int N>
-int launch(const M2NOp* ops, const uint32_t* tile_start, uint32_t n_ops, uint32_t grid, uint32_t* sync, const uint64_t* signals,
-           uint32_t n_signals, uint32_t epoch, int do_signal, cudaStream_t stream) {
-  if constexpr (has_instance(S, D, N)) {
-    m2n_typed_kernel<S, D, N><<<grid, kTypedThreads, 0, stream>>>(ops, tile_start, n_ops, sync, signals, n_signals, epoch, do_signal);
-    return 0;
-  } else {
-    return -1;
-  }
-}
-
-template <int S, int D>
-int by_nsrc(int n, const M2NOp* ops, const uint32_t* ts, uint32_t n_ops, uint32_t grid, uint32_t* sync, const uint64_t* sig,
-            uint32_t n_sig, uint32_t epoch, int do_signal, cudaStream_t st) {
-  switch (n) {
-    case 1: return launch<S, D, 1>(ops, ts, n_ops, grid, sync, sig, n_sig, epoch, do_signal, st);
-    case 2: return launch<S, D, 2>(ops, ts, n_ops, grid, sync, sig, n_sig, epoch, do_signal, st);
-    case 4: return launch<S, D, 4>(ops, ts, n_ops, grid, sync, sig, n_sig, epoch, do_signal, st);
-    default: return -1;
-  }
-}
-
-template <int S>
-int by_dst(int d, int n, const M2NOp* ops, const uint32_t* ts, uint32_t n_ops, uint32_t grid, uint32_t* sync, const uint64_t* sig,
-           uint32_t n_sig, uint32_t epoch, int do_signal, cudaStream_t st) {
-  switch (d) {
-    case M2N_F32: return by_nsrc<S, M2N_F32>(n, ops, ts, n_ops, grid, sync, sig, n_sig, epoch, do_signal, st);
-    case M2N_BF16: return by_nsrc<S, M2N_BF16>(n, ops, ts, n_ops, grid, sync, sig, n_sig, epoch, do_signal, st);
-    case M2N_F16: return by_nsrc<S, M2N_F16>(n, ops, ts, n_ops, grid, sync, sig, n_sig, epoch, do_signal, st);
-    default: return -1;
-  }
+int launch(const M2NLaunch& args, uint32_t grid, void* stream) {
+  if constexpr (has_instance(S, D, N)) return m2n_launch(m2n_typed_kernel<S, D, N>, grid, kTypedThreads, 0, stream, args, "typed");
+  else return m2n_no_instance("streaming", (S << 8) | (D << 4) | N);
 }
 
 }  // namespace
@@ -287,57 +256,31 @@ int etha_op_collapse_key(const M2NOp* op) {
   return M2N_KEY_COLLAPSE | ((op->red_size[1] > 1) << 8) | (op->src_dtype << 4) | op->dst_dtype;
 }
 
-int etha_m2n_collapse_launch(const M2NOp* ops, const uint32_t* tile_start, uint32_t n_ops, int key, uint32_t n_tiles,
-                             uint32_t* sync_scratch, const uint64_t* signals, uint32_t n_signals, uint32_t epoch, int do_signal,
-                             void* stream) {
-  if (!n_tiles) return 0;
-  cudaStream_t st = (cudaStream_t)stream;
-#define CASE_N(S, D, N)                                                                                                   \
-  case (N << 8) | (S << 4) | D:                                                                                           \
-    m2n_collapse_kernel<S, D, N><<<n_tiles, kTypedThreads, 0, st>>>(ops, tile_start, n_ops, sync_scratch, signals, n_signals, \
-                                                                    epoch, do_signal);                                    \
-    break;
+}  // extern "C"
+
+int m2n_launch_collapse(const M2NLaunch& args, int key, uint32_t n_tiles, void* stream) {
+#define CASE_N(S, D, N) \
+  case (N << 8) | (S << 4) | D: return m2n_launch(m2n_collapse_kernel<S, D, N>, n_tiles, kTypedThreads, 0, stream, args, "collapse");
 #define CASE(S, D) CASE_N(S, D, 0) CASE_N(S, D, 1)
   switch (key & 0xfff) {
     CASE(M2N_F32, M2N_F32) CASE(M2N_F32, M2N_BF16) CASE(M2N_F32, M2N_F16)
     CASE(M2N_BF16, M2N_F32) CASE(M2N_BF16, M2N_BF16) CASE(M2N_BF16, M2N_F16)
     CASE(M2N_F16, M2N_F32) CASE(M2N_F16, M2N_BF16) CASE(M2N_F16, M2N_F16)
-    default:
-      snprintf(etha_err_buf(), ETHA_ERR_LEN, "no collapse kernel instance for key 0x%x", key);
-      return -102;
+    default: return m2n_no_instance("collapse", key);
   }
 #undef CASE
 #undef CASE_N
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) {
-    snprintf(etha_err_buf(), ETHA_ERR_LEN, "collapse kernel launch: %s", cudaGetErrorString(e));
-    return -(int)e - 1000;
-  }
-  return 0;
 }
 
-int etha_m2n_typed_launch(const M2NOp* ops, const uint32_t* tile_start, uint32_t n_ops, int key, uint32_t n_tiles, uint32_t* sync_scratch,
-                          const uint64_t* signals, uint32_t n_signals, uint32_t epoch, int do_signal, void* stream) {
-  const int s = (key >> 8) & 0xf, d = (key >> 4) & 0xf, n = key & 0xf;
-  if (!n_tiles) return 0;
-  cudaStream_t st = (cudaStream_t)stream;
-  int rc;
-  switch (s) {
-    case M2N_F32: rc = by_dst<M2N_F32>(d, n, ops, tile_start, n_ops, n_tiles, sync_scratch, signals, n_signals, epoch, do_signal, st); break;
-    case M2N_BF16: rc = by_dst<M2N_BF16>(d, n, ops, tile_start, n_ops, n_tiles, sync_scratch, signals, n_signals, epoch, do_signal, st); break;
-    case M2N_F16: rc = by_dst<M2N_F16>(d, n, ops, tile_start, n_ops, n_tiles, sync_scratch, signals, n_signals, epoch, do_signal, st); break;
-    default: rc = -1;
+int m2n_launch_typed(const M2NLaunch& args, int key, uint32_t n_tiles, void* stream) {
+#define CASE_N(S, D, N) case (S << 8) | (D << 4) | N: return launch<S, D, N>(args, n_tiles, stream);
+#define CASE(S, D) CASE_N(S, D, 1) CASE_N(S, D, 2) CASE_N(S, D, 4)
+  switch (key) {
+    CASE(M2N_F32, M2N_F32) CASE(M2N_F32, M2N_BF16) CASE(M2N_F32, M2N_F16)
+    CASE(M2N_BF16, M2N_F32) CASE(M2N_BF16, M2N_BF16) CASE(M2N_BF16, M2N_F16)
+    CASE(M2N_F16, M2N_F32) CASE(M2N_F16, M2N_BF16) CASE(M2N_F16, M2N_F16)
+    default: return m2n_no_instance("streaming", key);
   }
-  if (rc != 0) {
-    snprintf(etha_err_buf(), ETHA_ERR_LEN, "no streaming kernel instance for key 0x%x", key);
-    return -102;
-  }
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) {
-    snprintf(etha_err_buf(), ETHA_ERR_LEN, "typed kernel launch: %s", cudaGetErrorString(e));
-    return -(int)e - 1000;
-  }
-  return 0;
+#undef CASE
+#undef CASE_N
 }
-
-}  // extern "C"

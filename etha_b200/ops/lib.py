@@ -15,8 +15,8 @@ MAX_DIMS = 4
 DT_RAW, DT_F32, DT_BF16, DT_F16 = 0, 1, 2, 3
 RED_CODES = {"sum": 0, "avg": 1, "max": 2, "min": 3, "product": 4}
 FLAG_MULTIMEM = 1
-# instance keys: the kernel's name by `key >> 12`
-INSTANCE_KERNELS = {0: "typed", 1: "ragged", 2: "collapse", 3: "transpose"}
+# kernel keys: below KEY_RAGGED a streaming instance, else the family and its fields
+KEY_RAGGED, KEY_COLLAPSE, KEY_TRANSPOSE, KEY_FAST, KEY_GENERAL, KEY_BULK = (f << 12 for f in range(1, 7))
 STATUS_OK, STATUS_TIMEOUT, STATUS_BAD_OP = 0, 1, 2
 
 
@@ -43,6 +43,11 @@ class OpSpec(C.Structure):
         ("flags", C.c_int32),
         ("tile_bytes", C.c_int32),
     ]
+
+
+class Launch(C.Structure):
+    _fields_ = [("key", C.c_int32), ("n_ops", C.c_uint32), ("n_tiles", C.c_uint32), ("pad", C.c_uint32),
+                ("ops", C.c_uint64), ("tiles", C.c_uint64)]
 
 
 class DmaCopy(C.Structure):
@@ -79,16 +84,14 @@ def cuda_lib() -> C.CDLL:
         lib.etha_m2n_run_noalloc.restype = i32
         lib.etha_m2n_noalloc_status.argtypes = [C.POINTER(u32), vp]
         lib.etha_m2n_noalloc_status.restype = i32
-        lib.etha_op_stream_key.argtypes = [vp]
-        lib.etha_op_stream_key.restype = i32
-        lib.etha_m2n_typed_launch.argtypes = [vp, vp, u32, i32, u32, vp, vp, u32, u32, i32, vp]
-        lib.etha_m2n_typed_launch.restype = i32
-        for name in ("ragged", "collapse", "transpose"):
-            key_of, launch = getattr(lib, f"etha_op_{name}_key"), getattr(lib, f"etha_m2n_{name}_launch")
-            key_of.argtypes, key_of.restype = [vp], i32
-            launch.argtypes, launch.restype = [vp, vp, u32, i32, u32, vp, vp, u32, u32, i32, vp], i32
-        lib.etha_m2n_launch.argtypes = [vp, vp, u32, i32, u32, i32, vp, vp, u32, u32, i32, vp]
-        lib.etha_m2n_launch.restype = i32
+        lib.etha_op_kernel_key.argtypes = [vp]
+        lib.etha_op_kernel_key.restype = i32
+        lib.etha_key_tile_class.argtypes = [i32]
+        lib.etha_key_tile_class.restype = i32
+        lib.etha_run.argtypes = [vp, u32, vp, vp, u32, u32, i32, vp]
+        lib.etha_run.restype = i32
+        lib.etha_run_spec.argtypes = [C.POINTER(OpSpec), vp]
+        lib.etha_run_spec.restype = i32
         lib.etha_set_flags.argtypes = [vp, u32, u32, vp]
         lib.etha_set_flags.restype = i32
         lib.etha_wait_flags.argtypes = [vp, vp, u32, u32, u64, vp, vp]
@@ -115,9 +118,6 @@ def cuda_lib() -> C.CDLL:
         lib.etha_enable_peer_access.restype = i32
         lib.etha_device_info.argtypes = [C.POINTER(i32)] * 4
         lib.etha_device_info.restype = i32
-        if hasattr(lib, "etha_m2n_bulk_launch"):
-            lib.etha_m2n_bulk_launch.argtypes = [vp, vp, u32, u32, vp, vp, u32, u32, i32, vp]
-            lib.etha_m2n_bulk_launch.restype = i32
         _lib = lib
         return lib
 

@@ -31,6 +31,13 @@ LAUNCH_COUNT = [0]
 DMA_COPY_COUNT = [0]
 
 
+def raw_stream(stream: torch.cuda.Stream | None, device: torch.device) -> int:
+    """Handle of `stream`, or of the device's current stream (read without building a Stream object)."""
+    if stream is not None:
+        return stream.cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if device.index is None else device.index)
+
+
 def dtype_code(dt: torch.dtype) -> int:
     return _DT_CODE.get(dt, L.DT_RAW)
 
@@ -52,21 +59,49 @@ class SliceRef:
         return SliceRef(view.data_ptr(), tuple(view.stride()), view.dtype, base, base + st.nbytes())
 
 
+def make_spec(shape, srcs, dsts, reduce_sizes, reduce_ops, flags: int, tile_bytes: int) -> L.OpSpec:
+    """Native description of one op; the slices of either side share strides and dtype."""
+    spec = L.OpSpec()
+    src0, dst0 = srcs[0], dsts[0]
+    n = spec.ndim = len(shape)
+    spec.shape[:n], spec.src_stride[:n], spec.dst_stride[:n] = shape, src0.strides[:n], dst0.strides[:n]
+    spec.src_itemsize, spec.dst_itemsize = src0.dtype.itemsize, dst0.dtype.itemsize
+    spec.src_dtype, spec.dst_dtype = dtype_code(src0.dtype), dtype_code(dst0.dtype)
+    if spec.src_dtype == L.DT_RAW and spec.dst_dtype == L.DT_RAW and src0.dtype != dst0.dtype:
+        raise ValueError(f"no conversion from {src0.dtype} to {dst0.dtype}")
+    spec.nsrc, spec.ndst = len(srcs), len(dsts)
+    for i, s in enumerate(srcs):
+        spec.src[i], spec.src_lo[i], spec.src_hi[i] = s.ptr, s.lo, s.hi
+    for i, d in enumerate(dsts):
+        spec.dst[i], spec.dst_lo[i], spec.dst_hi[i] = d.ptr, d.lo, d.hi
+    sizes = list(reduce_sizes) or [len(srcs)]
+    ops = list(reduce_ops) or ["sum"]
+    spec.red_size[0], spec.red_size[1] = sizes[0], (sizes[1] if len(sizes) > 1 else 1)
+    spec.red_op[0] = L.RED_CODES[ops[0]]
+    spec.red_op[1] = L.RED_CODES[ops[1]] if len(ops) > 1 else 0
+    spec.flags, spec.tile_bytes = flags, tile_bytes
+    return spec
+
+
 class _KernelSet:
-    """Launches that run one set of ops: `[(kernel, ops address, tile table address, number of ops, tiles), ...]`, without
-    and with the TMA kernel.  Until the table is uploaded the addresses are offsets into its buffer."""
+    """Launches that run one set of ops, without and with the TMA kernel.  Until the table is uploaded their addresses are
+    offsets into its buffer."""
 
     def __init__(self):
         self.n_ops, self.n_tiles = [0, 0], [0, 0]  # [fast class, general class]
         self.n_typed_ops = self.n_typed_tiles = 0
         self.n_bulk_ops = self.n_bulk_tiles = 0
-        self.ldst: list[tuple] = []
-        self.bulk: list[tuple] = []
+        self.ldst: list[L.Launch] = []
+        self.bulk: list[L.Launch] = []
 
-    def at(self, base: int) -> "_KernelSet":
+    def at(self, base: int) -> None:
+        """Make the launch lists what the native runner takes: (array of launches, its address, its length)."""
         for name in ("ldst", "bulk"):
-            setattr(self, name, [(k, base + ops, base + tiles, n, t) for k, ops, tiles, n, t in getattr(self, name)])
-        return self
+            launches = (L.Launch * len(getattr(self, name)))(*getattr(self, name))
+            for one in launches:
+                one.ops += base
+                one.tiles += base
+            setattr(self, name, (launches, C.addressof(launches), len(launches)))
 
 
 class _Blob:
@@ -110,6 +145,7 @@ class CopyTable:
         self._dma_plan = None
         self.dma_bytes = 0
         self._lib = L.cuda_lib()
+        self._run = self._lib.etha_run
         self._op_size = self._lib.etha_sizeof_op()
         self._packed: list[tuple[int, int, bytes, bool, int]] = []  # (class, tiles, op bytes, TMA-capable, instance key)
         # conversions / collapses over simple boxes use the streaming kernel instances, rows of any alignment the ragged ones
@@ -156,28 +192,7 @@ class CopyTable:
         for (dstrides, ddtype), members in groups.items():
             for k in range(0, len(members), L.MAX_DST):
                 part = members[k : k + L.MAX_DST]
-                spec = L.OpSpec()
-                spec.ndim = len(shape)
-                for i, n in enumerate(shape):
-                    spec.shape[i] = int(n)
-                    spec.src_stride[i] = int(src0.strides[i])
-                    spec.dst_stride[i] = int(dstrides[i])
-                spec.src_itemsize, spec.dst_itemsize = src0.dtype.itemsize, ddtype.itemsize
-                spec.src_dtype, spec.dst_dtype = dtype_code(src0.dtype), dtype_code(ddtype)
-                if spec.src_dtype == L.DT_RAW and spec.dst_dtype == L.DT_RAW and src0.dtype != ddtype:
-                    raise ValueError(f"no conversion from {src0.dtype} to {ddtype}")
-                spec.nsrc, spec.ndst = len(srcs), len(part)
-                for i, s in enumerate(srcs):
-                    spec.src[i], spec.src_lo[i], spec.src_hi[i] = s.ptr, s.lo, s.hi
-                for i, d in enumerate(part):
-                    spec.dst[i], spec.dst_lo[i], spec.dst_hi[i] = d.ptr, d.lo, d.hi
-                sizes = list(reduce_sizes) or [len(srcs)]
-                ops = list(reduce_ops) or ["sum"]
-                spec.red_size[0], spec.red_size[1] = sizes[0], (sizes[1] if len(sizes) > 1 else 1)
-                spec.red_op[0] = L.RED_CODES[ops[0]]
-                spec.red_op[1] = L.RED_CODES[ops[1]] if len(ops) > 1 else 0
-                spec.flags = L.FLAG_MULTIMEM if multimem else 0
-                spec.tile_bytes = self.tile_bytes
+                spec = make_spec(shape, srcs, part, reduce_sizes, reduce_ops, L.FLAG_MULTIMEM if multimem else 0, self.tile_bytes)
                 buf = C.create_string_buffer(self._op_size)
                 err = C.create_string_buffer(512)
                 rc = self._lib.etha_pack_op(C.byref(spec), buf, err, 512)
@@ -187,10 +202,10 @@ class CopyTable:
                 if tiles:
                     cls = self._lib.etha_op_class(buf)
                     tma = cls == 0 and bool(self._lib.etha_op_bulk_ok(buf))
-                    skey = 0
+                    skey = 0  # key of the kernel instance, 0: general kernel
                     if cls == 1 and self.stream_typed:
-                        skey = (self._lib.etha_op_stream_key(buf) or self._lib.etha_op_collapse_key(buf)
-                                or self._lib.etha_op_ragged_key(buf) or self._lib.etha_op_transpose_key(buf))
+                        skey = self._lib.etha_op_kernel_key(buf)
+                        skey = 0 if skey == L.KEY_GENERAL else skey
                     entry = (cls, tiles, buf.raw, tma, skey)
                     self._packed.append(entry)
                     if dma_ok and self.dma_min_bytes is not None and numel * ddtype.itemsize >= self.dma_min_bytes:
@@ -222,36 +237,37 @@ class CopyTable:
         """Put one set of packed ops into `blob`, split into the launches of the kernel classes."""
         ks = _KernelSet()
 
-        def launch(kernel, members, tile_class):
+        def launch(key, members):
             """One launch: tile sizes chosen for its kernel."""
             ops_host = np.frombuffer(b"".join(members), dtype=np.uint8).copy()
             starts = np.zeros(len(members) + 1, dtype=np.uint32)
-            tiles = self._lib.etha_layout_tiles(ops_host.ctypes.data, len(members), tile_class, starts.ctypes.data)
+            tiles = self._lib.etha_layout_tiles(ops_host.ctypes.data, len(members), self._lib.etha_key_tile_class(key),
+                                                starts.ctypes.data)
             if tiles < 0:
                 raise ValueError("too many tiles in one table")
-            return kernel, blob.add(ops_host), blob.add(starts), len(members), tiles
+            return L.Launch(key, len(members), tiles, 0, blob.add(ops_host), blob.add(starts))
 
         rest = []  # launches of the typed and general classes
         for key in dict.fromkeys(k for c, _, _, _, k in packed if c == 1 and k):
-            kernel = L.INSTANCE_KERNELS[key >> 12]
-            rest.append(launch(key, [raw for c, _, raw, _, k in packed if c == 1 and k == key], {"ragged": 2, "transpose": 3}.get(kernel, 0)))
-            if kernel == "typed":
-                ks.n_typed_ops += rest[-1][3]
-                ks.n_typed_tiles += rest[-1][4]
+            one = launch(key, [raw for c, _, raw, _, k in packed if c == 1 and k == key])
+            rest.append(one)
+            if key < L.KEY_RAGGED:
+                ks.n_typed_ops += one.n_ops
+                ks.n_typed_tiles += one.n_tiles
             else:
-                ks.n_ops[1] += rest[-1][3]
-                ks.n_tiles[1] += rest[-1][4]
+                ks.n_ops[1] += one.n_ops
+                ks.n_tiles[1] += one.n_tiles
         general = [raw for c, _, raw, _, k in packed if c == 1 and not k]
         if general:
-            rest.append(launch("general", general, 1))
-            ks.n_ops[1] += rest[-1][3]
-            ks.n_tiles[1] += rest[-1][4]
+            rest.append(launch(L.KEY_GENERAL, general))
+            ks.n_ops[1] += rest[-1].n_ops
+            ks.n_tiles[1] += rest[-1].n_tiles
         fast = [(t, raw, tma) for c, t, raw, tma, _ in packed if c == 0]
         if fast:
             # stable split: TMA-capable ops first, relative order kept inside both groups
             tma, other = [m for m in fast if m[2]], [m for m in fast if not m[2]]
-            ks.ldst.append(launch("fast", [raw for _, raw, _ in tma + other], 0))
-            ks.n_ops[0], ks.n_tiles[0] = ks.ldst[0][3:]
+            ks.ldst.append(launch(L.KEY_FAST, [raw for _, raw, _ in tma + other]))
+            ks.n_ops[0], ks.n_tiles[0] = ks.ldst[0].n_ops, ks.ldst[0].n_tiles
             if tma:
                 # the TMA kernel cuts its tiles into ring stages and keeps the table's tile size
                 starts = np.zeros(len(tma) + 1, dtype=np.uint64)
@@ -259,10 +275,10 @@ class CopyTable:
                 if starts[-1] >= 2**31:
                     raise ValueError("too many tiles in one table")
                 ks.n_bulk_ops, ks.n_bulk_tiles = len(tma), int(starts[-1])
-                ks.bulk.append(("bulk", blob.add(np.frombuffer(b"".join(raw for _, raw, _ in tma), dtype=np.uint8)),
-                                blob.add(starts.astype(np.uint32)), len(tma), ks.n_bulk_tiles))
+                ops_at = blob.add(np.frombuffer(b"".join(raw for _, raw, _ in tma), dtype=np.uint8))
+                ks.bulk.append(L.Launch(L.KEY_BULK, len(tma), ks.n_bulk_tiles, 0, ops_at, blob.add(starts.astype(np.uint32))))
                 if other:
-                    ks.bulk.append(launch("fast", [raw for _, raw, _ in other], 0))
+                    ks.bulk.append(launch(L.KEY_FAST, [raw for _, raw, _ in other]))
             else:
                 ks.bulk = list(ks.ldst)
         ks.ldst += rest
@@ -299,6 +315,7 @@ class CopyTable:
         self._rest = self._lay_out([e for i, e in enumerate(self._packed) if i not in taken], blob) if taken else self._all
         self._buffer = blob.upload(self.device)
         self._sync = self._buffer[:16].view(torch.int32)
+        self._sync_ptr = self._buffer.data_ptr()
         for ks in {id(k): k for k in (self._all, self._rest)}.values():
             ks.at(self._buffer.data_ptr())
         # [fast class, typed + general]: the streaming instances count with the general class they were taken from
@@ -353,42 +370,31 @@ class CopyTable:
         the kernels even if the table holds a DMA plan."""
         if not self._final:
             self.finalize()
-        s = (stream or torch.cuda.current_stream(self.device)).cuda_stream
-        n_sig = 0 if signals is None else signals.numel()
-        sig_ptr = 0 if signals is None else signals.data_ptr()
+        s = raw_stream(stream, self.device)
+        sig_ptr, n_sig = (0, 0) if signals is None else (signals.data_ptr(), signals.numel())
         dma = self._dma_plan is not None and dma is not False
         ks = self._rest if dma else self._all
-        plan = ks.bulk if bulk else ks.ldst
-        if not plan or dma:
-            # with DMA copies in the transfer: the copies start on side streams, the kernels run next to them on
-            # the caller's stream without a signal, the stream then waits for the copies and the flags go last
-            if dma:
-                L.check(self._lib.etha_dma_plan_launch(self._dma_plan, s), "dma launch")
-                DMA_COPY_COUNT[0] += len(self._dma)
-            for kernel, ops_ptr, tiles_ptr, n_ops, n_tiles in plan:
-                self._launch_kernel(kernel, ops_ptr, tiles_ptr, n_ops, n_tiles, ctas_per_sm, (sig_ptr, 0, 0, 0), s)
-            if dma:
-                L.check(self._lib.etha_dma_plan_join(self._dma_plan, s), "dma join")
-            if n_sig:
-                L.check(self._lib.etha_set_flags(sig_ptr, n_sig, epoch & 0xFFFFFFFF, s), "set_flags")
-                LAUNCH_COUNT[0] += 1
+        _, launches, n = ks.bulk if bulk else ks.ldst
+        epoch &= 0xFFFFFFFF
+        if n and not dma:
+            rc = self._run(launches, n, self._sync_ptr, sig_ptr, n_sig, epoch, ctas_per_sm, s)
+            if rc:
+                L.check(rc, "m2n launch")
+            LAUNCH_COUNT[0] += n
             return
-        for i, (kernel, ops_ptr, tiles_ptr, n_ops, n_tiles) in enumerate(plan):
-            last = i == len(plan) - 1
-            sig = (sig_ptr, n_sig, epoch & 0xFFFFFFFF, 1) if (last and n_sig) else (sig_ptr, 0, epoch & 0xFFFFFFFF, 0)
-            self._launch_kernel(kernel, ops_ptr, tiles_ptr, n_ops, n_tiles, ctas_per_sm, sig, s)
-
-    def _launch_kernel(self, kernel, ops_ptr, tiles_ptr, n_ops, n_tiles, ctas_per_sm, sig, s) -> None:
-        if kernel == "bulk":
-            rc = self._lib.etha_m2n_bulk_launch(ops_ptr, tiles_ptr, n_ops, n_tiles, self._sync.data_ptr(), *sig, s)
-        elif isinstance(kernel, int):  # key of an instance
-            launch = getattr(self._lib, f"etha_m2n_{L.INSTANCE_KERNELS[kernel >> 12]}_launch")
-            rc = launch(ops_ptr, tiles_ptr, n_ops, kernel, n_tiles, self._sync.data_ptr(), *sig, s)
-        else:
-            rc = self._lib.etha_m2n_launch(ops_ptr, tiles_ptr, n_ops, int(kernel == "general"), n_tiles, ctas_per_sm,
-                                           self._sync.data_ptr(), *sig, s)
-        L.check(rc, "m2n launch")
-        LAUNCH_COUNT[0] += 1
+        # with DMA copies in the transfer: the copies start on side streams, the kernels run next to them on
+        # the caller's stream without a signal, the stream then waits for the copies and the flags go last
+        if dma:
+            L.check(self._lib.etha_dma_plan_launch(self._dma_plan, s), "dma launch")
+            DMA_COPY_COUNT[0] += len(self._dma)
+        if n:
+            L.check(self._run(launches, n, self._sync_ptr, 0, 0, epoch, ctas_per_sm, s), "m2n launch")
+            LAUNCH_COUNT[0] += n
+        if dma:
+            L.check(self._lib.etha_dma_plan_join(self._dma_plan, s), "dma join")
+        if n_sig:
+            L.check(self._lib.etha_set_flags(sig_ptr, n_sig, epoch, s), "set_flags")
+            LAUNCH_COUNT[0] += 1
 
     def error_word(self) -> int:
         """Device-side error word of the last launches (synchronizes)."""

@@ -15,22 +15,42 @@ from dataclasses import dataclass
 import torch
 
 
-@contextlib.contextmanager
-def nvtx_range(name: str):
-    """NVTX range + torch.profiler record_function around a block (plan / launch / wait phases)."""
-    pushed = False
-    if torch.cuda.is_available():
-        try:
-            torch.cuda.nvtx.range_push(name)
-            pushed = True
-        except Exception:
-            pushed = False
-    try:
-        with torch.profiler.record_function(name):
-            yield
-    finally:
-        if pushed:
+def _profiler_on() -> bool:
+    """Whether a torch profiler of any kind is recording in this process or thread."""
+    return torch.autograd.profiler._is_profiler_enabled or torch.autograd._profiler_enabled()
+
+
+class nvtx_range:
+    """NVTX range + torch.profiler record_function around a block (plan / launch / wait phases).  The record_function,
+    which costs more than the launch it surrounds, is opened only while a profiler records."""
+
+    _nvtx: bool | None = None  # whether this process can push NVTX ranges
+
+    def __init__(self, name: str):
+        self.name = name
+
+    def __enter__(self):
+        cls = nvtx_range
+        self.pushed = False
+        if cls._nvtx is not False:
+            try:
+                if cls._nvtx or torch.cuda.is_available():
+                    torch.cuda.nvtx.range_push(self.name)
+                    self.pushed = cls._nvtx = True
+                else:
+                    cls._nvtx = False
+            except Exception:
+                cls._nvtx = False
+        self.record = torch.profiler.record_function(self.name) if _profiler_on() else None
+        if self.record is not None:
+            self.record.__enter__()
+
+    def __exit__(self, *exc):
+        if self.record is not None:
+            self.record.__exit__(*exc)
+        if self.pushed:
             torch.cuda.nvtx.range_pop()
+        return False
 
 
 @dataclass
