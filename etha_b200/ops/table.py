@@ -2,9 +2,9 @@
 
 `CopyTable.add*` collect strided-box copies (optionally converting, fanning out to several
 destinations or collapsing several Partial sources); `finalize()` packs them with the native packer,
-splits them into the two kernel classes and uploads them; `launch()` issues at most two persistent
-kernels on the given stream and, when asked, publishes an epoch to the consumers' flags from the
-last CTA.  Nothing here allocates or touches the host during `launch()`.
+splits them by the kernel that runs them and uploads them in one copy; `launch()` issues one kernel per group on
+the given stream in one native call and, when asked, publishes an epoch to the consumers' flags after the
+last tile.  Nothing here allocates or touches the host during `launch()`.
 
 The reference does this work per chunk and per transfer in Python (`Chunk.prepare`/`Bucket.prepare`/
 `finalize`, src/etha/comm/ir.py:101-141,229-310).
@@ -125,7 +125,9 @@ class _Blob:
 
 
 class CopyTable:
-    """`dma_min_bytes`: when set, a bit copy of at least that many bytes whose box is one run or the rows of a matrix,
+    """`tile_bytes`: upper bound of a tile (destination bytes); the TMA kernel uses it as it is, the others cut finer.
+
+    `dma_min_bytes`: when set, a bit copy of at least that many bytes whose box is one run or the rows of a matrix,
     and which the caller marks `dma_ok` (its destination is on another GPU), is a candidate for the DMA engines: at
     `finalize()` the largest candidates, up to `dma_fraction` of the bytes the table delivers, become memcpy nodes
     of a CUDA graph (`dma_mode="graph"`) or asynchronous copies on `dma_streams` side streams
