@@ -154,6 +154,7 @@ m2n_bulk_kernel(const __grid_constant__ M2NLaunch args) {
     }
   }
   sched_init(&ring.sched);
+  after_previous_kernel();
 
   if (threadIdx.x < 32) {
     // ---- load warp --------------------------------------------------------------------------------------
@@ -221,10 +222,8 @@ m2n_bulk_kernel(const __grid_constant__ M2NLaunch args) {
     asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     asm volatile("fence.proxy.async;" ::: "memory");
   }
-  if (args.do_signal) {
-    __syncthreads();
-    finish_and_signal(args, s_done);
-  }
+  __syncthreads();
+  finish(args, s_done);
 }
 
 }  // namespace

@@ -17,13 +17,15 @@ namespace {
 // ---------------------------------------------------------------------------------------------
 // memory access helpers
 // ---------------------------------------------------------------------------------------------
+// (plain loads, not the non-coherent ones: the sources may be written by the kernel before this one while this one is
+// already resident, see `after_previous_kernel`; both kinds run at the same speed)
 template <typename V>
 __device__ __forceinline__ V ld_stream(const void* p);
 
 template <>
 __device__ __forceinline__ uint4 ld_stream<uint4>(const void* p) {
   uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
                : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                : "l"(p));
   return v;
@@ -31,25 +33,25 @@ __device__ __forceinline__ uint4 ld_stream<uint4>(const void* p) {
 template <>
 __device__ __forceinline__ uint2 ld_stream<uint2>(const void* p) {
   uint2 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+  asm volatile("ld.global.L1::no_allocate.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
   return v;
 }
 template <>
 __device__ __forceinline__ uint32_t ld_stream<uint32_t>(const void* p) {
   uint32_t v;
-  asm volatile("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  asm volatile("ld.global.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));
   return v;
 }
 template <>
 __device__ __forceinline__ uint16_t ld_stream<uint16_t>(const void* p) {
   uint16_t v;
-  asm volatile("ld.global.nc.L1::no_allocate.u16 %0, [%1];" : "=h"(v) : "l"(p));
+  asm volatile("ld.global.L1::no_allocate.u16 %0, [%1];" : "=h"(v) : "l"(p));
   return v;
 }
 template <>
 __device__ __forceinline__ uint8_t ld_stream<uint8_t>(const void* p) {
   uint32_t v;
-  asm volatile("ld.global.nc.L1::no_allocate.u8 %0, [%1];" : "=r"(v) : "l"(p));
+  asm volatile("ld.global.L1::no_allocate.u8 %0, [%1];" : "=r"(v) : "l"(p));
   return (uint8_t)v;
 }
 
@@ -57,7 +59,7 @@ __device__ __forceinline__ uint8_t ld_stream<uint8_t>(const void* p) {
 // first load allocate the sector in L1 so that the second one does not go back to L2
 __device__ __forceinline__ uint4 ld_keep(const void* p) {
   uint4 v;
-  asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
 }
 
@@ -361,6 +363,16 @@ __device__ __forceinline__ void sched_locate(TileSched* s, const M2NLaunch& args
   __syncthreads();
 }
 
+// Waits until the kernel before this one in the stream has finished and its writes are visible.  EVERY thread of EVERY kernel
+// launched as a dependent passes here before it touches anything that is not its own launch's table: a kernel that
+// finishes has then also outwaited all kernels before its predecessor.
+__device__ __forceinline__ void after_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Lets the next kernel in the stream start its set-up once every CTA has come here (or ended).  One thread calls it, after a
+// barrier of its CTA and a fence: a kernel that reads weights ahead of its own wait, because it takes them for
+// constants, then still finds what this one has delivered.
+__device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Walk over all tiles of the table: `body(op, first unit, one past the last unit)` runs with all threads of the CTA.
 // Returns the number of tiles this CTA ran.  CHUNKS: the tiles are counted in the op's chunks instead of its units.
 template <bool CHUNKS = false, typename Body>
@@ -370,6 +382,7 @@ __device__ __forceinline__ uint32_t for_each_tile(TileSched* s, M2NOp* s_op, con
   while (true) {
     if (threadIdx.x == 0) sched_request(s);
     sched_locate(s, args, tile, s_op);
+    if (!done) after_previous_kernel();
     const M2NOp& op = *s_op;
     const uint32_t base = (tile - s->begin) * op.tile_units;
     body(op, base, min(CHUNKS ? op.chunks : op.total_units, base + op.tile_units));
@@ -386,11 +399,15 @@ __device__ __forceinline__ uint32_t for_each_tile(TileSched* s, M2NOp* s_op, con
 // its system-scope release stores order them for the consumers too (release patterns are cumulative).  What a small table
 // of 592 CTAs pays for its signal: 13 us with a system-scope fence in every CTA, 5 us with a GPU-scope one there and a
 // system-scope fence before the release stores, 3 us as it stands.
-__device__ __forceinline__ void finish_and_signal(const M2NLaunch& args, uint32_t done) {
+__device__ __forceinline__ void finish(const M2NLaunch& args, uint32_t done) {
   __shared__ uint32_t s_last;
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
+    let_next_kernel_start();
+  }
+  if (!args.do_signal) return;
+  if (threadIdx.x == 0) {
     const uint32_t prev = atomicAdd(&args.sync[0], done);
     s_last = (prev + done == gridDim.x) ? 1u : 0u;
     __threadfence();

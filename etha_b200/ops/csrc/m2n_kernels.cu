@@ -1,7 +1,7 @@
 // sm_100a kernels of the M-to-N redistribution: strided gather -> (convert | reduce) -> strided
 // scatter into local, peer or multicast memory, plus the release/acquire flag kernels.
 //
-// One persistent launch walks a device-resident table of `M2NOp`s (see m2n.h).  The table is built
+// A launch walks a device-resident table of `M2NOp`s (see m2n.h).  The table is built
 // once per registered batch and launched once per transfer, so a transfer costs no host work per
 // chunk and no staging buffer: the producer GPU reads its own memory and stores straight into the
 // consumers' slices over NVLink.  This replaces the reference's per-chunk slice/contiguous/cast/
@@ -305,7 +305,7 @@ m2n_fast_kernel(const __grid_constant__ M2NLaunch args) {
     if (op.ndim == 0) fast_tile<0>(op, base, limit);
     else fast_tile<1>(op, base, limit);
   });
-  if (args.do_signal) finish_and_signal(args, done);
+  finish(args, done);
 }
 
 // General class: any other bit copy, converting copies and Partial collapses.
@@ -333,7 +333,7 @@ m2n_general_kernel(const __grid_constant__ M2NLaunch args) {
       if (threadIdx.x == 0) report(args, M2N_BAD_OP);
     }
   });
-  if (args.do_signal) finish_and_signal(args, done);
+  finish(args, done);
 }
 
 __global__ void set_flags_kernel(const uint64_t* __restrict__ signals, uint32_t n_signals, uint32_t epoch) {
@@ -344,36 +344,45 @@ __global__ void set_flags_kernel(const uint64_t* __restrict__ signals, uint32_t 
   }
 }
 
-// Bounded acquire-wait.  A flag counts as set once it reached `epoch` (wrap-safe compare).  On timeout the
-// kernel reports which flag was missing and returns; it never traps and never spins without a limit.
-__global__ void wait_flags_kernel(const uint32_t* __restrict__ flags, const uint32_t* __restrict__ which, uint32_t n,
-                                  uint32_t epoch, uint64_t timeout_ns, uint32_t* status) {
-  __shared__ uint32_t s_fail, s_who;
-  if (threadIdx.x == 0) { s_fail = 0; s_who = 0xffffffffu; }
-  __syncthreads();
-  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+// Bounded acquire-wait by one warp.  A flag counts as set once it reached `epoch` (wrap-safe compare).  On timeout the
+// kernel reports which flag was missing and returns; it never traps and never spins without a limit.  It lets the
+// next kernel of the stream start only when it has seen the flags: CTAs that are resident while it spins could keep a
+// producer off this GPU.  What it costs when the flags are set already is latency only: the clock is read after the first
+// miss, and both status words go out in one store where their address allows it.
+__global__ void __launch_bounds__(32)
+wait_flags_kernel(const uint32_t* __restrict__ flags, const uint32_t* __restrict__ which, uint32_t n, uint32_t epoch,
+                  uint64_t timeout_ns, uint32_t* status) {
+  after_previous_kernel();
+  uint32_t missing = 0xffffffffu;
+  for (uint32_t i = threadIdx.x; i < n; i += 32) {
     const uint32_t* flag = flags + which[i];
-    uint64_t t0;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
+    uint64_t t0 = 0;
     bool ok = false;
     for (uint64_t it = 0; it < (1ull << 34); ++it) {
       uint32_t v;
       asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(flag) : "memory");
       if ((int32_t)(v - epoch) >= 0) { ok = true; break; }
-      if ((it & 63) == 63) {
+      if ((it & 63) == 0) {
         uint64_t t;
         asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-        if (t - t0 > timeout_ns) break;
-        __nanosleep(200);
+        if (it == 0) t0 = t;
+        else if (t - t0 > timeout_ns) break;
+        else __nanosleep(200);
       }
     }
-    if (!ok) { atomicExch(&s_fail, 1u); atomicMin(&s_who, i); }
+    if (!ok) missing = min(missing, i);
   }
-  __syncthreads();
+  missing = __reduce_min_sync(0xffffffffu, missing);
   if (threadIdx.x == 0) {
-    status[1] = s_who;
-    __threadfence_system();
-    status[0] = s_fail ? M2N_TIMEOUT : M2N_OK;
+    let_next_kernel_start();
+    const uint32_t code = missing == 0xffffffffu ? M2N_OK : M2N_TIMEOUT;
+    if ((reinterpret_cast<uint64_t>(status) & 7) == 0) {
+      *reinterpret_cast<uint2*>(status) = make_uint2(code, missing);
+    } else {
+      status[1] = missing;
+      __threadfence_system();
+      status[0] = code;
+    }
   }
 }
 
@@ -406,9 +415,8 @@ int etha_set_flags(const uint64_t* signals, uint32_t n_signals, uint32_t epoch, 
 
 int etha_wait_flags(const uint32_t* flags, const uint32_t* which, uint32_t n, uint32_t epoch, uint64_t timeout_ns,
                     uint32_t* status, void* stream) {
-  int block = n < 32 ? 32 : (n > 256 ? 256 : (int)((n + 31) & ~31u));
-  wait_flags_kernel<<<1, block, 0, (cudaStream_t)stream>>>(flags, which, n, epoch, timeout_ns, status);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = m2n_launch_dependent(wait_flags_kernel, 1, 32, 0, stream, flags, which, n, epoch, timeout_ns, status);
+  if (e != cudaSuccess) cudaGetLastError();
   return e == cudaSuccess ? 0 : fail(e, "wait_flags launch");
 }
 

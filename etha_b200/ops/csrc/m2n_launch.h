@@ -21,11 +21,28 @@ struct M2NLaunch {
   M2NOp one;
 };
 
+// Launch as a programmatic dependent of the kernel before it in the stream: the CTAs may become resident, set up their
+// queue and fetch their op while that kernel finishes; everything else comes after `after_previous_kernel`.
+template <typename Kernel, typename... Args>
+inline cudaError_t m2n_launch_dependent(Kernel kernel, uint32_t grid, int block, size_t smem, void* stream, Args... args) {
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(grid);
+  config.blockDim = dim3(block);
+  config.dynamicSmemBytes = smem;
+  config.stream = (cudaStream_t)stream;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = &attr;
+  config.numAttrs = 1;
+  return cudaLaunchKernelEx(&config, kernel, args...);
+}
+
 template <typename Kernel>
 inline int m2n_launch(Kernel kernel, uint32_t grid, int block, size_t smem, void* stream, const M2NLaunch& args, const char* what) {
-  kernel<<<grid, block, smem, (cudaStream_t)stream>>>(args);
-  const cudaError_t e = cudaGetLastError();
+  const cudaError_t e = m2n_launch_dependent(kernel, grid, block, smem, stream, args);
   if (e == cudaSuccess) return 0;
+  cudaGetLastError();
   snprintf(etha_err_buf(), ETHA_ERR_LEN, "%s kernel launch: %s", what, cudaGetErrorString(e));
   return -(int)e - 1000;
 }

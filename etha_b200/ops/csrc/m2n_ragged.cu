@@ -33,7 +33,7 @@ constexpr int kRaggedUnroll = 2;
 
 __device__ __forceinline__ uint4 ld_word(const char* p) {  // aligned 16 bytes, kept in L1 for the neighbouring chunk
   uint4 v;
-  asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];"
+  asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];"
                : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                : "l"(__cvta_generic_to_global(p)));
   return v;
@@ -270,7 +270,7 @@ m2n_ragged_kernel(const __grid_constant__ M2NLaunch args) {
 #pragma unroll 1
     for (b += threadIdx.x; b < limit; b += kRaggedThreads) trip(std::integral_constant<int, 1>(), b);
   });
-  if (args.do_signal) finish_and_signal(args, done);
+  finish(args, done);
 }
 
 }  // namespace

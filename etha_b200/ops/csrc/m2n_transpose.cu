@@ -198,7 +198,7 @@ m2n_transpose_kernel(const __grid_constant__ M2NLaunch args) {
     }
     for (uint32_t b = base; b < limit; ++b) block_move<SDT, DDT, ES>(op, b, s_tile);
   });
-  if (args.do_signal) finish_and_signal(args, done);
+  finish(args, done);
 }
 
 }  // namespace

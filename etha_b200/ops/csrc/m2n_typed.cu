@@ -104,7 +104,7 @@ m2n_typed_kernel(const __grid_constant__ M2NLaunch args) {
     if (op.ndim == 0) stream_tile<SDT, DDT, NSRC, 0>(op, base, limit);
     else stream_tile<SDT, DDT, NSRC, 1>(op, base, limit);
   });
-  if (args.do_signal) finish_and_signal(args, done);
+  finish(args, done);
 }
 
 // Collapses without an instance of their own (3 or 5 to 8 sources, two levels, the two 16-bit types mixed): one kernel per
@@ -211,7 +211,7 @@ m2n_collapse_kernel(const __grid_constant__ M2NLaunch args) {
 #pragma unroll 1
     for (b += threadIdx.x; b < limit; b += kTypedThreads) collapse_trip<SDT, DDT, TWO, 1>(op, b);
   });
-  if (args.do_signal) finish_and_signal(args, done);
+  finish(args, done);
 }
 
 constexpr bool typed(int dt) { return dt == M2N_F32 || dt == M2N_BF16 || dt == M2N_F16; }
