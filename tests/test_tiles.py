@@ -82,3 +82,42 @@ def test_two_streams_share_a_table():
             marks.append((dst == src).all())  # what this stream sees after its own launch
     torch.cuda.synchronize()
     assert all(bool(m) for m in marks)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("n", [8, 100_003, 4_000_000])
+def test_chained_launches_see_each_other(graph, n):
+    """A kernel that is resident before its predecessor ends still reads what that one, and the ones before it, wrote."""
+    dev = torch.device("cuda", 0)
+    bufs = [torch.zeros(n + 1, dtype=torch.int32, device=dev)[i % 2 :][:n] for i in range(12)]  # aligned and not
+    tables = []
+    for src, dst in zip(bufs, bufs[1:]):
+        t = CopyTable(dev)
+        t.add_copy(src, dst)
+        tables.append(t.finalize())
+    stream = torch.cuda.Stream(dev)
+    start = torch.zeros(1, dtype=torch.int32, device=dev)
+
+    def chain():
+        start.add_(1)
+        bufs[0].copy_(start.expand(n))
+        for t in tables:
+            t.launch(stream)
+        return bufs[-1] + 0  # what the next kernel in the stream sees
+
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        out = chain()
+        if graph:
+            torch.cuda.synchronize()
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=stream):
+                out = chain()
+        for k in range(2, 12):
+            if graph:
+                g.replay()
+            else:
+                out = chain()
+            stream.synchronize()
+            assert bool((out == k).all()), k
