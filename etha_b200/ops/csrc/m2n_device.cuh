@@ -87,22 +87,29 @@ __device__ __forceinline__ void st_multimem16(void* p, uint4 v) {
                : "memory");
 }
 
-__device__ __forceinline__ uint32_t fast_div(uint32_t n, uint32_t mul, uint32_t shr) {
+__host__ __device__ __forceinline__ uint32_t fast_div(uint32_t n, uint32_t mul, uint32_t shr) {
+#ifdef __CUDA_ARCH__
   return mul ? (__umulhi(n, mul) >> shr) : n;  // mul == 0 encodes "divide by one"
+#else
+  return mul ? (uint32_t)(((uint64_t)n * mul) >> 32) >> shr : n;
+#endif
 }
 
-// byte offsets of unit `unit` of the op inside the source and the destination box
-template <int ND = -1>
-__device__ __forceinline__ void unit_offsets(const M2NOp& op, uint32_t unit, int64_t& so, int64_t& dof) {
+// byte offsets of unit `unit` of the op inside the source and the destination box; BYTES: size of a unit on both sides
+// where the kernel knows it.  A row can be longer than 4 GiB (28 bits of 16-byte units): bytes are 64 bits wide
+// throughout.  The host runs the same code in etha_op_unit_offsets.
+template <int ND = -1, int BYTES = 0>
+__host__ __device__ __forceinline__ void unit_offsets(const M2NOp& op, uint32_t unit, int64_t& so, int64_t& dof) {
+  const uint32_t bytes_src = BYTES ? BYTES : op.unit_bytes_src, bytes_dst = BYTES ? BYTES : op.unit_bytes_dst;
   if constexpr (ND == 0) {  // one contiguous run on both sides
-    so = (int64_t)unit * op.unit_bytes_src;
-    dof = (int64_t)unit * op.unit_bytes_dst;
+    so = (int64_t)unit * bytes_src;
+    dof = (int64_t)unit * bytes_dst;
     return;
   }
   uint32_t q = fast_div(unit, op.div_mul[M2N_MAX_DIMS], op.div_shr[M2N_MAX_DIMS]);
   uint32_t col = unit - q * op.inner_units;
-  so = (int64_t)col * op.unit_bytes_src;
-  dof = (int64_t)col * op.unit_bytes_dst;
+  so = (int64_t)col * bytes_src;
+  dof = (int64_t)col * bytes_dst;
   if constexpr (ND == 1) {  // rows of a matrix
     so += (int64_t)q * op.src_stride[0];
     dof += (int64_t)q * op.dst_stride[0];

@@ -246,7 +246,7 @@ __device__ __forceinline__ bool dispatch_typed(const M2NOp& op, uint32_t base, u
 }
 
 // Fast class: 16-byte bit copies whose box is one run or rows of a matrix (the bulk of a weight sync).  Bound by HBM (or
-// NVLink): 4 x 512 threads per SM at 30 registers, two 16-byte loads each before the first store, tiles of one such trip
+// NVLink): 4 x 512 threads per SM at 32 registers, two 16-byte loads each before the first store, tiles of one such trip
 // (16 KiB).  1 GiB on one GPU, read + written: contiguous 6.72 TB/s, 2 KiB rows out of 8 KiB ones 6.45, one source and four
 // destinations 6.51 (2 x 512 threads with four loads and a fixed stride of 64 KiB tiles: 5.52, 5.79, 5.37).  With 76 bytes of
 // spills per thread the same kernel falls to 5.97, so full trips carry no per-unit predicate.
@@ -262,16 +262,9 @@ __device__ __forceinline__ void fast_trip(const M2NOp& op, uint32_t unit0) {
   const char* src = reinterpret_cast<const char*>(op.src[0]);
 #pragma unroll
   for (int u = 0; u < U; ++u) {
-    if constexpr (ND == 0) {
-      dof[u] = (int64_t)unit0 * 16 + u * kFastThreads * 16;
-      v[u] = ld_stream<uint4>(src + dof[u]);
-    } else {
-      const uint32_t unit = unit0 + u * kFastThreads;
-      const uint32_t q = fast_div(unit, op.div_mul[M2N_MAX_DIMS], op.div_shr[M2N_MAX_DIMS]);
-      const uint32_t col = (unit - q * op.inner_units) * 16;
-      dof[u] = col + (int64_t)q * op.dst_stride[0];
-      v[u] = ld_stream<uint4>(src + col + (int64_t)q * op.src_stride[0]);
-    }
+    int64_t so;
+    unit_offsets<ND, 16>(op, unit0 + u * kFastThreads, so, dof[u]);
+    v[u] = ld_stream<uint4>(src + so);
   }
   if (op.flags & M2N_FLAG_MULTIMEM) {
 #pragma unroll

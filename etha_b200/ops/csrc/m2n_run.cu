@@ -1,6 +1,7 @@
 // Entry points that run launches: a table's list of them, and copies whose ops travel in the kernel arguments.
 #include <cstring>
 
+#include "m2n_device.cuh"
 #include "m2n_launch.h"
 
 extern "C" {
@@ -21,6 +22,12 @@ int etha_key_tile_class(int key) {
     case M2N_KEY_TRANSPOSE >> 12: return 3;
     default: return 0;
   }
+}
+
+void etha_op_unit_offsets(const M2NOp* op, uint32_t unit, int64_t* src, int64_t* dst) {
+  if (etha_op_class(op) != 0) unit_offsets(*op, unit, *src, *dst);
+  else if (op->ndim == 0) unit_offsets<0, 16>(*op, unit, *src, *dst);
+  else unit_offsets<1, 16>(*op, unit, *src, *dst);
 }
 
 }  // extern "C"

@@ -80,6 +80,8 @@ def cuda_lib() -> C.CDLL:
         lib.etha_layout_tiles.restype = C.c_int64
         lib.etha_op_bulk_ok.argtypes = [vp]
         lib.etha_op_bulk_ok.restype = i32
+        lib.etha_op_unit_offsets.argtypes = [vp, u32, C.POINTER(C.c_int64), C.POINTER(C.c_int64)]
+        lib.etha_op_unit_offsets.restype = None
         lib.etha_m2n_run_noalloc.argtypes = [C.POINTER(OpSpec), u32, i32, vp]
         lib.etha_m2n_run_noalloc.restype = i32
         lib.etha_m2n_noalloc_status.argtypes = [C.POINTER(u32), vp]
