@@ -13,7 +13,8 @@
 // with 16-byte aligned bases and strides into this class.  A side that is contiguous over the whole fill is
 // moved with ONE bulk copy per stage instead of one per matrix row.
 // Waits on the barriers are bounded: after the limit the warp records an error word, drains its own stores
-// and returns; the other warp runs into its own limit.
+// and returns; the other warp runs into its own limit.  Tiles given up count as finished, and the error word keeps the
+// flags back.
 //
 // 1 GiB on one GPU, read + written: contiguous 6.55 TB/s, 2 KiB rows out of 8 KiB ones 6.46, one source and four
 // destinations 6.46 (one warp for both directions and a fixed stride of tiles: 6.00, 5.42, 5.67).  Six stages of 32 KiB:
@@ -186,11 +187,15 @@ m2n_bulk_kernel(const __grid_constant__ M2NLaunch args) {
           ++fills;
         }
       }
-      ++done;
-      const bool more = sched_take(&ring.sched, phase, tile, args);
+      ++done;  // run or given up: see `finish`
+      const Take take = sched_take(&ring.sched, phase, tile, args);
+      if (__any_sync(0xffffffffu, take == kGaveUp)) {
+        done += sched_abandon(&ring.sched, phase);
+        break;
+      }
       phase ^= 1;
-      __syncwarp();
-      alive = alive && more;
+      if (!alive) done += take == kTile;  // taken over, but this CTA has stopped
+      alive = alive && take == kTile;
     }
     if (stage_free() && lane == 0) {  // end mark
       ring.meta[fills % kStages].npieces = 0;

@@ -399,5 +399,6 @@ class CopyTable:
             LAUNCH_COUNT[0] += 1
 
     def error_word(self) -> int:
-        """Device-side error word of the last launches (synchronizes)."""
+        """Device-side error word (synchronizes): 0, or the status bits of every failure since `finalize()`.  A table
+        whose word is set publishes no epoch any more; it has to be built again."""
         return int(self._sync[1].item()) if (self.n_tiles[0] + self.n_tiles[1]) else 0
