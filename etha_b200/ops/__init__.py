@@ -27,8 +27,20 @@ __all__ = [
 ]
 
 
+def _reachable(src: torch.Tensor, device: torch.device) -> None:
+    """Raise unless kernels on `device` can read `src`: its address goes into the launch as it is."""
+    if src.is_cuda:
+        if src.device != device:
+            with torch.cuda.device(device):
+                if cuda_lib().etha_enable_peer_access(src.device.index):
+                    raise ValueError(f"{device} cannot read the memory of {src.device}: {_L.last_error()}")
+    elif not src.is_pinned():
+        raise ValueError(f"the source must be on a CUDA device or in pinned host memory, not on {src.device}")
+
+
 def local_copy(src: torch.Tensor, dst: torch.Tensor, stream: torch.cuda.Stream | None = None) -> None:
-    """`dst[...] = src` (any strides, fp32/bf16/fp16 conversion) through the copy kernels."""
+    """`dst[...] = src` (any strides, fp32/bf16/fp16 conversion) through the copy kernels.  `dst` is on a CUDA device, `src`
+    on the same one, on a peer of it or in pinned host memory."""
     shape = tuple(src.shape)
     if shape != tuple(dst.shape):
         raise ValueError(f"shape mismatch {shape} vs {tuple(dst.shape)}")
@@ -40,6 +52,7 @@ def local_copy(src: torch.Tensor, dst: torch.Tensor, stream: torch.cuda.Stream |
     spec = make_spec(shape, [SliceRef.of(src)], [SliceRef.of(dst)], (), (), 0, 0)
     if not src.numel():
         return
+    _reachable(src, dst.device)
     rc = cuda_lib().etha_run_spec(_byref(spec), raw_stream(stream, dst.device))
     if -100 < rc < 0:  # refused by the packer
         raise ValueError(f"cannot pack op ({rc}): {_L.last_error()}")
