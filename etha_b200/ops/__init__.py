@@ -8,7 +8,7 @@ import torch
 
 from . import lib as _L
 from .lib import STATUS_BAD_OP, STATUS_OK, STATUS_TIMEOUT, cuda_lib
-from .table import LAUNCH_COUNT, CopyTable, SliceRef, dtype_code, make_spec, raw_stream
+from .table import LAUNCH_COUNT, CopyTable, SliceRef, device_index, dtype_code, make_spec, raw_stream
 
 FLAG_LAUNCH_COUNT = [0]  # set_flags / wait_flags kernels launched in this process
 
@@ -28,12 +28,11 @@ __all__ = [
 
 
 def _reachable(src: torch.Tensor, device: torch.device) -> None:
-    """Raise unless kernels on `device` can read `src`: its address goes into the launch as it is."""
+    """Raise unless kernels on `device` can read `src`, which is not there: its address goes into the launch as it is."""
     if src.is_cuda:
-        if src.device != device:
-            with torch.cuda.device(device):
-                if cuda_lib().etha_enable_peer_access(src.device.index):
-                    raise ValueError(f"{device} cannot read the memory of {src.device}: {_L.last_error()}")
+        with torch.cuda.device(device):
+            if cuda_lib().etha_enable_peer_access(src.device.index):
+                raise ValueError(f"{device} cannot read the memory of {src.device}: {_L.last_error()}")
     elif not src.is_pinned():
         raise ValueError(f"the source must be on a CUDA device or in pinned host memory, not on {src.device}")
 
@@ -52,8 +51,11 @@ def local_copy(src: torch.Tensor, dst: torch.Tensor, stream: torch.cuda.Stream |
     spec = make_spec(shape, [SliceRef.of(src)], [SliceRef.of(dst)], (), (), 0, 0)
     if not src.numel():
         return
-    _reachable(src, dst.device)
-    rc = cuda_lib().etha_run_spec(_byref(spec), raw_stream(stream, dst.device))
+    index = dst.get_device()
+    if src.get_device() != index:
+        _reachable(src, dst.device)
+    s = torch._C._cuda_getCurrentRawStream(index) if stream is None else stream.cuda_stream
+    rc = cuda_lib().etha_run_spec(_byref(spec), index, s)
     if -100 < rc < 0:  # refused by the packer
         raise ValueError(f"cannot pack op ({rc}): {_L.last_error()}")
     _L.check(rc, "local copy")
@@ -62,8 +64,10 @@ def local_copy(src: torch.Tensor, dst: torch.Tensor, stream: torch.cuda.Stream |
 
 def set_flags(addresses: torch.Tensor, epoch: int, stream: torch.cuda.Stream | None = None) -> None:
     """Store `epoch` (release, system scope) to every uint32 flag whose address is in `addresses` (int64, device)."""
-    s = raw_stream(stream, addresses.device)
-    _L.check(cuda_lib().etha_set_flags(addresses.data_ptr(), addresses.numel(), epoch & 0xFFFFFFFF, s), "set_flags")
+    device = addresses.device
+    rc = cuda_lib().etha_set_flags(addresses.data_ptr(), addresses.numel(), epoch & 0xFFFFFFFF, device_index(device),
+                                   raw_stream(stream, device))
+    _L.check(rc, "set_flags")
     FLAG_LAUNCH_COUNT[0] += 1
 
 
@@ -80,8 +84,9 @@ def wait_flags(
     `status` (int32[2], device or pinned-mapped) receives `[STATUS_OK | STATUS_TIMEOUT, index of the
     first missing flag]`.  The wait gives up after `timeout_s`; the context stays usable.
     """
+    device = flags.device
     rc = cuda_lib().etha_wait_flags(flags.data_ptr(), which.data_ptr(), which.numel(), epoch & 0xFFFFFFFF, int(timeout_s * 1e9),
-                                    status.data_ptr(), raw_stream(stream, flags.device))
+                                    status.data_ptr(), device_index(device), raw_stream(stream, device))
     if rc:
         _L.check(rc, "wait_flags")
     FLAG_LAUNCH_COUNT[0] += 1

@@ -379,10 +379,7 @@ wait_flags_kernel(const uint32_t* __restrict__ flags, const uint32_t* __restrict
   }
 }
 
-inline int fail(cudaError_t e, const char* what) {
-  snprintf(etha_err_buf(), ETHA_ERR_LEN, "%s: %s", what, cudaGetErrorString(e));
-  return -(int)e - 1000;
-}
+inline int fail(cudaError_t e, const char* what) { return m2n_cuda_error(e, what); }
 
 }  // namespace
 
@@ -400,14 +397,18 @@ int m2n_launch_copy(const M2NLaunch& args, bool general, uint32_t n_tiles, int c
 
 extern "C" {
 
-int etha_set_flags(const uint64_t* signals, uint32_t n_signals, uint32_t epoch, void* stream) {
+int etha_set_flags(const uint64_t* signals, uint32_t n_signals, uint32_t epoch, int device, void* stream) {
+  const OnDevice on(device);
+  if (on.error != cudaSuccess) return fail(on.error, "device of the launch");
   set_flags_kernel<<<1, 64, 0, (cudaStream_t)stream>>>(signals, n_signals, epoch);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : fail(e, "set_flags launch");
 }
 
 int etha_wait_flags(const uint32_t* flags, const uint32_t* which, uint32_t n, uint32_t epoch, uint64_t timeout_ns,
-                    uint32_t* status, void* stream) {
+                    uint32_t* status, int device, void* stream) {
+  const OnDevice on(device);
+  if (on.error != cudaSuccess) return fail(on.error, "device of the launch");
   cudaError_t e = m2n_launch_dependent(wait_flags_kernel, 1, 32, 0, stream, flags, which, n, epoch, timeout_ns, status);
   if (e != cudaSuccess) cudaGetLastError();
   return e == cudaSuccess ? 0 : fail(e, "wait_flags launch");
@@ -513,7 +514,7 @@ extern "C" int etha_m2n_run_noalloc(const M2NOpSpec* specs, uint32_t n_specs, in
     if (e != cudaSuccess) return fail(e, "cudaMemcpyAsync(tile table)");
     e = cudaMemcpyAsync(class_ops, packed[c], count[c] * sizeof(M2NOp), cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) return fail(e, "cudaMemcpyAsync(op table)");
-    const EthaLaunch launch = {c == 0 ? M2N_KEY_FAST : M2N_KEY_GENERAL, count[c], tile_start[c][count[c]], 0,
+    const EthaLaunch launch = {c == 0 ? M2N_KEY_FAST : M2N_KEY_GENERAL, count[c], tile_start[c][count[c]], dev,
                                reinterpret_cast<uint64_t>(class_ops), reinterpret_cast<uint64_t>(tiles_dev)};
     rc = etha_run(&launch, 1, reinterpret_cast<uint32_t*>(scratch + 256 * c), nullptr, 0, 0, ctas_per_sm, s);
     if (rc != 0) return rc;

@@ -21,6 +21,29 @@ struct M2NLaunch {
   M2NOp one;
 };
 
+// Makes `device` current while it lives (-1: leaves the current one). `error`: why it could not.
+struct OnDevice {
+  int before = -1;
+  cudaError_t error;
+  explicit OnDevice(int device) {
+    int now = -1;
+    error = cudaGetDevice(&now);
+    if (error != cudaSuccess || device < 0 || device == now) return;
+    error = cudaSetDevice(device);
+    if (error == cudaSuccess) before = now;
+    else cudaGetLastError();  // not the error of the next call
+  }
+  ~OnDevice() {
+    if (before >= 0) cudaSetDevice(before);
+  }
+  OnDevice(const OnDevice&) = delete;
+};
+
+inline int m2n_cuda_error(cudaError_t e, const char* what) {
+  snprintf(etha_err_buf(), ETHA_ERR_LEN, "%s: %s", what, cudaGetErrorString(e));
+  return -(int)e - 1000;
+}
+
 // Launch as a programmatic dependent of the kernel before it in the stream: the CTAs may become resident, set up their
 // queue and fetch their op while that kernel finishes; everything else comes after `after_previous_kernel`.
 template <typename Kernel, typename... Args>

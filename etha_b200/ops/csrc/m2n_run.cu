@@ -58,6 +58,9 @@ int etha_run(const EthaLaunch* launches, uint32_t n, uint32_t* sync, const uint6
   args.sync = sync;
   args.signals = signals;
   args.epoch = epoch;
+  if (!n) return 0;
+  const OnDevice on(launches[0].device);
+  if (on.error != cudaSuccess) return m2n_cuda_error(on.error, "device of the launch");
   for (uint32_t i = 0; i < n; ++i) {
     const EthaLaunch& l = launches[i];
     args.ops = reinterpret_cast<const M2NOp*>(l.ops);
@@ -72,7 +75,7 @@ int etha_run(const EthaLaunch* launches, uint32_t n, uint32_t* sync, const uint6
   return 0;
 }
 
-int etha_run_spec(const M2NOpSpec* spec, void* stream) {
+int etha_run_spec(const M2NOpSpec* spec, int device, void* stream) {
   M2NLaunch args;
   memset(&args, 0, sizeof(args));
   const int rc = etha_pack_op(spec, &args.one, nullptr, 0);
@@ -86,6 +89,8 @@ int etha_run_spec(const M2NOpSpec* spec, void* stream) {
     return -101;
   }
   args.n_ops = 1;
+  const OnDevice on(device);
+  if (on.error != cudaSuccess) return m2n_cuda_error(on.error, "device of the launch");
   return run_one(args, key, (uint32_t)tiles, 0, stream);
 }
 

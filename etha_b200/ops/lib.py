@@ -46,7 +46,7 @@ class OpSpec(C.Structure):
 
 
 class Launch(C.Structure):
-    _fields_ = [("key", C.c_int32), ("n_ops", C.c_uint32), ("n_tiles", C.c_uint32), ("pad", C.c_uint32),
+    _fields_ = [("key", C.c_int32), ("n_ops", C.c_uint32), ("n_tiles", C.c_uint32), ("device", C.c_int32),
                 ("ops", C.c_uint64), ("tiles", C.c_uint64)]
 
 
@@ -92,11 +92,11 @@ def cuda_lib() -> C.CDLL:
         lib.etha_key_tile_class.restype = i32
         lib.etha_run.argtypes = [vp, u32, vp, vp, u32, u32, i32, vp]
         lib.etha_run.restype = i32
-        lib.etha_run_spec.argtypes = [C.POINTER(OpSpec), vp]
+        lib.etha_run_spec.argtypes = [C.POINTER(OpSpec), i32, vp]
         lib.etha_run_spec.restype = i32
-        lib.etha_set_flags.argtypes = [vp, u32, u32, vp]
+        lib.etha_set_flags.argtypes = [vp, u32, u32, i32, vp]
         lib.etha_set_flags.restype = i32
-        lib.etha_wait_flags.argtypes = [vp, vp, u32, u32, u64, vp, vp]
+        lib.etha_wait_flags.argtypes = [vp, vp, u32, u32, u64, vp, i32, vp]
         lib.etha_wait_flags.restype = i32
         lib.etha_ipc_export.argtypes = [u64, C.c_char_p, C.POINTER(u64), C.POINTER(u64)]
         lib.etha_ipc_export.restype = i32

@@ -38,6 +38,11 @@ def raw_stream(stream: torch.cuda.Stream | None, device: torch.device) -> int:
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if device.index is None else device.index)
 
 
+def device_index(device: torch.device) -> int:
+    """What the launching entries of the library take: -1 stands for whatever device is current."""
+    return -1 if device.index is None else device.index
+
+
 def dtype_code(dt: torch.dtype) -> int:
     return _DT_CODE.get(dt, L.DT_RAW)
 
@@ -238,6 +243,7 @@ class CopyTable:
     def _lay_out(self, packed, blob: _Blob) -> "_KernelSet":
         """Put one set of packed ops into `blob`, split into the launches of the kernel classes."""
         ks = _KernelSet()
+        device = device_index(self.device)
 
         def launch(key, members):
             """One launch: tile sizes chosen for its kernel."""
@@ -247,7 +253,7 @@ class CopyTable:
                                                 starts.ctypes.data)
             if tiles < 0:
                 raise ValueError("too many tiles in one table")
-            return L.Launch(key, len(members), tiles, 0, blob.add(ops_host), blob.add(starts))
+            return L.Launch(key, len(members), tiles, device, blob.add(ops_host), blob.add(starts))
 
         rest = []  # launches of the typed and general classes
         for key in dict.fromkeys(k for c, _, _, _, k in packed if c == 1 and k):
@@ -278,7 +284,7 @@ class CopyTable:
                     raise ValueError("too many tiles in one table")
                 ks.n_bulk_ops, ks.n_bulk_tiles = len(tma), int(starts[-1])
                 ops_at = blob.add(np.frombuffer(b"".join(raw for _, raw, _ in tma), dtype=np.uint8))
-                ks.bulk.append(L.Launch(L.KEY_BULK, len(tma), ks.n_bulk_tiles, 0, ops_at, blob.add(starts.astype(np.uint32))))
+                ks.bulk.append(L.Launch(L.KEY_BULK, len(tma), ks.n_bulk_tiles, device, ops_at, blob.add(starts.astype(np.uint32))))
                 if other:
                     ks.bulk.append(launch(L.KEY_FAST, [raw for _, raw, _ in other]))
             else:
@@ -306,6 +312,8 @@ class CopyTable:
     def finalize(self, sm_count: int | None = None) -> "CopyTable":
         if self._final:
             return self
+        if self.device.type == "cuda" and self.device.index is None:  # the table lives on one device from here on
+            self.device = torch.device("cuda", torch.cuda.current_device())
         if sm_count is None:
             sm_count = torch.cuda.get_device_properties(self.device).multi_processor_count
         self.sm_count = sm_count
@@ -387,15 +395,17 @@ class CopyTable:
         # with DMA copies in the transfer: the copies start on side streams, the kernels run next to them on
         # the caller's stream without a signal, the stream then waits for the copies and the flags go last
         if dma:
-            L.check(self._lib.etha_dma_plan_launch(self._dma_plan, s), "dma launch")
+            with torch.cuda.device(self.device):
+                L.check(self._lib.etha_dma_plan_launch(self._dma_plan, s), "dma launch")
             DMA_COPY_COUNT[0] += len(self._dma)
         if n:
             L.check(self._run(launches, n, self._sync_ptr, 0, 0, epoch, ctas_per_sm, s), "m2n launch")
             LAUNCH_COUNT[0] += n
         if dma:
-            L.check(self._lib.etha_dma_plan_join(self._dma_plan, s), "dma join")
+            with torch.cuda.device(self.device):
+                L.check(self._lib.etha_dma_plan_join(self._dma_plan, s), "dma join")
         if n_sig:
-            L.check(self._lib.etha_set_flags(sig_ptr, n_sig, epoch, s), "set_flags")
+            L.check(self._lib.etha_set_flags(sig_ptr, n_sig, epoch, device_index(self.device), s), "set_flags")
             LAUNCH_COUNT[0] += 1
 
     def error_word(self) -> int:

@@ -1,9 +1,10 @@
-"""`local_copy`: what it refuses and where it launches."""
+"""`local_copy`: what it refuses; which device the launches go to."""
 
 import pytest
 import torch
 
 from etha_b200 import ops
+from etha_b200.ops.table import _Blob
 
 
 class _Cuda:
@@ -11,6 +12,9 @@ class _Cuda:
 
     def __init__(self, t, index=0):
         self._t, self.device, self.is_cuda = t, torch.device("cuda", index), True
+
+    def get_device(self):
+        return self.device.index
 
     def __getattr__(self, name):
         return getattr(self._t, name)
@@ -26,9 +30,18 @@ class _Lib:
     def __init__(self, peers=True):
         self.calls, self.peers = [], peers
 
-    def etha_run_spec(self, spec, stream):
-        self.calls.append(("run", stream))
+    def etha_run_spec(self, spec, device, stream):
+        self.calls.append(("run", stream, device))
         return 0
+
+    def etha_set_flags(self, addresses, n, epoch, device, stream):
+        self.calls.append(("set", stream, device))
+        return 0
+
+    def etha_wait_flags(self, flags, which, n, epoch, timeout, status, device, stream):
+        self.calls.append(("wait", stream, device))
+        return 0
+
 
     def etha_enable_peer_access(self, index):
         self.calls.append(("peer", index))
@@ -81,11 +94,42 @@ def test_a_host_destination_is_refused(lib):
 def test_a_source_on_another_gpu_needs_peer_access(lib):
     src, dst = _Cuda(torch.zeros(8), 1), _Cuda(torch.zeros(8), 0)
     ops.local_copy(src, dst, _Stream())
-    assert lib.calls == [("peer", 1), ("run", 77)]
+    assert lib.calls == [("peer", 1), ("run", 77, 0)]
     lib.calls, lib.peers = [], False
     with pytest.raises(ValueError, match="cuda:0 cannot read the memory of cuda:1"):
         ops.local_copy(src, dst, _Stream())
     assert lib.calls == [("peer", 1)]
+
+
+@pytest.mark.parametrize("index", [0, 1])
+def test_launches_go_to_the_device_of_their_memory(lib, index):
+    """Whatever device is current: a default stream has the same handle on all of them."""
+    x = _Cuda(torch.zeros(8), index)
+    ops.local_copy(x, _Cuda(torch.zeros(8), index), _Stream())
+    ops.set_flags(x, 1, _Stream())
+    ops.wait_flags(x, x, 1, x, 1.0, _Stream())
+    assert lib.calls == [(name, 77, index) for name in ("run", "set", "wait")]
+
+
+@pytest.mark.parametrize("device,index", [("cuda:0", 0), ("cuda:1", 1), ("cuda", -1)])
+def test_a_table_names_its_device_in_every_launch(device, index):
+    t = ops.CopyTable(torch.device("cpu"))  # packed and laid out on the host
+    t.device = torch.device(device)
+    for n, dtype in [(64, torch.float32), (16, torch.bfloat16), (7, torch.float32)]:
+        t.add((n,), [ops.SliceRef(1 << 30, (1,), torch.float32)], [ops.SliceRef(1 << 32, (1,), dtype)])
+    ks = t._lay_out(t._packed, _Blob())
+    assert len(ks.ldst) == 3 and len(ks.bulk) == 3
+    assert {one.device for one in ks.ldst + ks.bulk} == {index}
+
+
+@pytest.mark.gpu
+def test_an_unknown_device_is_an_error_and_the_current_one_stays():
+    x = torch.zeros(8, dtype=torch.int64, device="cuda:0")
+    lib, before = ops.cuda_lib(), torch.cuda.current_device()
+    assert lib.etha_set_flags(x.data_ptr(), 0, 1, torch.cuda.device_count(), 0) < 0
+    assert torch.cuda.current_device() == before
+    assert lib.etha_set_flags(x.data_ptr(), 0, 1, before, 0) == 0 and lib.etha_set_flags(x.data_ptr(), 0, 1, -1, 0) == 0
+    torch.cuda.synchronize()
 
 
 @pytest.mark.gpu
