@@ -37,9 +37,23 @@ def _reachable(src: torch.Tensor, device: torch.device) -> None:
         raise ValueError(f"the source must be on a CUDA device or in pinned host memory, not on {src.device}")
 
 
+def _after_current(stream: torch.cuda.Stream, index: int) -> int:
+    """Handle of `stream`, made to wait for the current stream of device `index`, which may still be writing the source."""
+    current = torch.cuda.current_stream(index)
+    with torch.cuda.stream(stream):
+        capturing = torch.cuda.is_current_stream_capturing()
+    if capturing:
+        with torch.cuda.stream(current):
+            if not torch.cuda.is_current_stream_capturing():
+                return stream.cuda_stream  # a graph cannot wait for work outside of it
+    stream.wait_stream(current)
+    return stream.cuda_stream
+
+
 def local_copy(src: torch.Tensor, dst: torch.Tensor, stream: torch.cuda.Stream | None = None) -> None:
     """`dst[...] = src` (any strides, fp32/bf16/fp16 conversion) through the copy kernels.  `dst` is on a CUDA device, `src`
-    on the same one, on a peer of it or in pinned host memory."""
+    on the same one, on a peer of it or in pinned host memory.  A copy on another `stream` than the device's current one
+    comes after what the current stream holds at the call; whoever uses `dst` elsewhere, or frees either tensor, waits for it."""
     shape = tuple(src.shape)
     if shape != tuple(dst.shape):
         raise ValueError(f"shape mismatch {shape} vs {tuple(dst.shape)}")
@@ -54,7 +68,9 @@ def local_copy(src: torch.Tensor, dst: torch.Tensor, stream: torch.cuda.Stream |
     index = dst.get_device()
     if src.get_device() != index:
         _reachable(src, dst.device)
-    s = torch._C._cuda_getCurrentRawStream(index) if stream is None else stream.cuda_stream
+    s = torch._C._cuda_getCurrentRawStream(index)
+    if stream is not None and stream.cuda_stream != s:
+        s = _after_current(stream, index)
     rc = cuda_lib().etha_run_spec(_byref(spec), index, s)
     if -100 < rc < 0:  # refused by the packer
         raise ValueError(f"cannot pack op ({rc}): {_L.last_error()}")

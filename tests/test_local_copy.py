@@ -1,4 +1,7 @@
-"""`local_copy`: what it refuses; which device the launches go to."""
+"""`local_copy`: what it refuses, which device the launches go to, what they come after."""
+
+from contextlib import nullcontext
+from types import SimpleNamespace
 
 import pytest
 import torch
@@ -73,6 +76,7 @@ def lib(monkeypatch):
     monkeypatch.setattr(ops._L, "cuda_lib", lambda: fake)
     monkeypatch.setattr(torch.cuda, "device", _Guard)
     monkeypatch.setattr(torch.cuda, "current_device", lambda: _Guard.now)
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda index: 77)
     return fake
 
 
@@ -130,6 +134,58 @@ def test_an_unknown_device_is_an_error_and_the_current_one_stays():
     assert torch.cuda.current_device() == before
     assert lib.etha_set_flags(x.data_ptr(), 0, 1, before, 0) == 0 and lib.etha_set_flags(x.data_ptr(), 0, 1, -1, 0) == 0
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("handle", [77, 78])
+def test_a_copy_on_another_stream_is_ordered(lib, monkeypatch, handle):
+    current, waits = object(), []
+    stream = SimpleNamespace(cuda_stream=handle, wait_stream=lambda other: waits.append((other, len(lib.calls))))
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda index: current)
+    monkeypatch.setattr(torch.cuda, "stream", lambda s: nullcontext())
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    ops.local_copy(_Cuda(torch.zeros(8)), _Cuda(torch.zeros(8)), stream)
+    assert waits == ([] if handle == 77 else [(current, 0)])  # before the launch
+    assert lib.calls == [("run", handle, 0)]
+
+
+@pytest.mark.gpu
+def test_another_stream_waits_for_the_current_one():
+    """The source is still being written on the current stream when the copy is put on a side stream."""
+    src = torch.zeros(1 << 20, dtype=torch.int32, device="cuda:0")
+    dst = torch.zeros_like(src)
+    side = torch.cuda.Stream("cuda:0")
+    torch.cuda.synchronize()
+    for k in range(1, 4):
+        torch.cuda._sleep(20_000_000)  # about 10 ms
+        src.fill_(k)
+        ops.local_copy(src, dst, side)
+        side.synchronize()
+        assert bool((dst == k).all())
+    torch.cuda.synchronize()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("forked", [False, True])
+def test_other_streams_under_capture(forked):
+    """Into a capturing stream that is not current, and from a capture into a stream forked off it."""
+    src = torch.arange(1000, dtype=torch.float32, device="cuda:0")
+    dst = torch.zeros_like(src)
+    one, two = torch.cuda.Stream("cuda:0"), torch.cuda.Stream("cuda:0")
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(one):
+        graph.capture_begin()
+        if forked:
+            ops.local_copy(src, dst, two)
+            one.wait_stream(two)
+        else:
+            with torch.cuda.stream(two):
+                ops.local_copy(src, dst, one)
+        graph.capture_end()
+    assert not dst.any()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(dst, src)
 
 
 @pytest.mark.gpu
