@@ -20,14 +20,17 @@ def _profiler_on() -> bool:
     return torch.autograd.profiler._is_profiler_enabled or torch.autograd._profiler_enabled()
 
 
-class nvtx_range:
-    """NVTX range + torch.profiler record_function around a block (plan / launch / wait phases).  The record_function,
-    which costs more than the launch it surrounds, is opened only while a profiler records."""
+class nvtx_range(contextlib.ContextDecorator):
+    """NVTX range + torch.profiler record_function around a block or a function (plan / launch / wait phases).  The
+    record_function, which costs more than the launch it surrounds, is opened only while a profiler records."""
 
     _nvtx: bool | None = None  # whether this process can push NVTX ranges
 
     def __init__(self, name: str):
         self.name = name
+
+    def _recreate_cm(self):  # calls of a decorated function may nest
+        return nvtx_range(self.name)
 
     def __enter__(self):
         cls = nvtx_range

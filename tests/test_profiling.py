@@ -30,3 +30,18 @@ def test_profiling_off_yields_none(tmp_path):
     with maybe_enable_profiling(ProfilingSpec(enable_profiling=False, dump_folder=str(tmp_path))) as prof:
         assert prof is None
     assert not os.listdir(tmp_path)
+
+
+def test_a_range_decorates_functions(monkeypatch):
+    """Every call opens a range of its own, nested calls among them."""
+    depth = []
+
+    @nvtx_range("etha.step")
+    def step(n):
+        depth.append(n)
+        return step(n - 1) + n if n else 0
+
+    with torch.profiler.profile() as prof:
+        assert step(3) == 6
+    assert depth == [3, 2, 1, 0]
+    assert [e.count for e in prof.key_averages() if e.key == "etha.step"] == [4]
