@@ -8,6 +8,7 @@ Counterpart of the reference's bench/utils.py:36-123 (`ProfilingSpec`, `maybe_en
 from __future__ import annotations
 
 import contextlib
+import ctypes
 import os
 import pickle
 from dataclasses import dataclass
@@ -15,16 +16,26 @@ from dataclasses import dataclass
 import torch
 
 
-def _profiler_on() -> bool:
-    """Whether a torch profiler of any kind is recording in this process or thread."""
-    return torch.autograd.profiler._is_profiler_enabled or torch.autograd._profiler_enabled()
+def _callback_query():
+    """`at::hasCallbacks`: whether anything in this process or thread observes record_function (the profilers, an execution
+    trace observer, a profiler started from outside).  torch has no Python name for it; it takes no arguments and is
+    called by its exported name.  Without it every range counts as observed."""
+    try:
+        query = ctypes.PyDLL(os.path.join(os.path.dirname(torch.__file__), "lib", "libtorch_cpu.so"))._ZN2at12hasCallbacksEv
+    except (OSError, AttributeError):
+        return lambda: True
+    query.argtypes, query.restype = [], ctypes.c_bool
+    return query
+
+
+_observed = _callback_query()
 
 
 class nvtx_range(contextlib.ContextDecorator):
     """NVTX range + torch.profiler record_function around a block or a function (plan / launch / wait phases).  The
-    record_function, which costs more than the launch it surrounds, is opened only while a profiler records."""
+    record_function, which costs more than the launch it surrounds, is opened only while somebody observes it."""
 
-    _nvtx: bool | None = None  # whether this process can push NVTX ranges
+    _nvtx = False  # an NVTX range has been pushed in this process
 
     def __init__(self, name: str):
         self.name = name
@@ -33,19 +44,15 @@ class nvtx_range(contextlib.ContextDecorator):
         return nvtx_range(self.name)
 
     def __enter__(self):
-        cls = nvtx_range
-        self.pushed = False
-        if cls._nvtx is not False:
-            try:
-                if cls._nvtx or torch.cuda.is_available():
-                    torch.cuda.nvtx.range_push(self.name)
-                    self.pushed = cls._nvtx = True
-                else:
-                    cls._nvtx = False
-            except Exception:
-                cls._nvtx = False
-        self.record = torch.profiler.record_function(self.name) if _profiler_on() else None
-        if self.record is not None:
+        self.record, self.pushed = None, False
+        try:
+            if nvtx_range._nvtx or torch.cuda.is_available():
+                torch.cuda.nvtx.range_push(self.name)
+                self.pushed = nvtx_range._nvtx = True
+        except Exception:
+            pass
+        if _observed():
+            self.record = torch.profiler.record_function(self.name)
             self.record.__enter__()
 
     def __exit__(self, *exc):

@@ -45,3 +45,38 @@ def test_a_range_decorates_functions():
         assert [step(0), step(0), step(3)] == [0, 0, 6]
     assert depth == [0, 0, 3, 2, 1, 0]
     assert [e.count for e in prof.key_averages() if e.key == "etha.step"] == [3]
+
+
+def test_other_observers_see_the_ranges(tmp_path):
+    """Not only the autograd profiler listens to record_function."""
+    path = str(tmp_path / "trace.json")
+    observer = torch.profiler.ExecutionTraceObserver().register_callback(path)
+    observer.start()
+    with nvtx_range("etha.observed"):
+        torch.zeros(1)
+    observer.stop()
+    with nvtx_range("etha.unobserved"):
+        torch.zeros(1)
+    observer.unregister_callback()
+    names = {n["name"] for n in json.load(open(path))["nodes"]}
+    assert "etha.observed" in names and "etha.unobserved" not in names
+
+
+def test_a_failed_push_does_not_turn_nvtx_off(monkeypatch):
+    pushed = []
+
+    def push(name):
+        if not pushed:
+            pushed.append(None)
+            raise RuntimeError("first push fails")
+        pushed.append(name)
+
+    monkeypatch.setattr(nvtx_range, "_nvtx", nvtx_range._nvtx)
+    monkeypatch.setattr(torch.cuda, "is_available", lambda: True)
+    monkeypatch.setattr(torch.cuda.nvtx, "range_push", push)
+    monkeypatch.setattr(torch.cuda.nvtx, "range_pop", lambda: pushed.pop())
+    with nvtx_range("a"):
+        assert pushed == [None]
+    with nvtx_range("b"):
+        assert pushed == [None, "b"]
+    assert pushed == [None]
