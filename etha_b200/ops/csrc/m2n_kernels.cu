@@ -337,33 +337,42 @@ __global__ void set_flags_kernel(const uint64_t* __restrict__ signals, uint32_t 
   }
 }
 
+__device__ __forceinline__ bool flag_is_set(const uint32_t* flag, uint32_t epoch) {
+  uint32_t v;
+  asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(flag) : "memory");
+  return (int32_t)(v - epoch) >= 0;
+}
+
 // Bounded acquire-wait by one warp.  A flag counts as set once it reached `epoch` (wrap-safe compare).  On timeout the
-// kernel reports which flag was missing and returns; it never traps and never spins without a limit.  It lets the
+// kernel reports which flag was missing and returns; it never traps and never spins without a limit.  All flags share one
+// deadline, however many of them a lane looks after.  It lets the
 // next kernel of the stream start only when it has seen the flags: CTAs that are resident while it spins could keep a
-// producer off this GPU.  What it costs when the flags are set already is latency only: the clock is read after the first
-// miss, and both status words go out in one store where their address allows it.
+// producer off this GPU.  What it costs when the flags are set already is latency only: the clock is read once a lane has
+// missed one, and both status words go out in one store where their address allows it.
 __global__ void __launch_bounds__(32)
 wait_flags_kernel(const uint32_t* __restrict__ flags, const uint32_t* __restrict__ which, uint32_t n, uint32_t epoch,
                   uint64_t timeout_ns, uint32_t* status) {
   after_previous_kernel();
   uint32_t missing = 0xffffffffu;
-  for (uint32_t i = threadIdx.x; i < n; i += 32) {
-    const uint32_t* flag = flags + which[i];
-    uint64_t t0 = 0;
-    bool ok = false;
-    for (uint64_t it = 0; it < (1ull << 34); ++it) {
-      uint32_t v;
-      asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(flag) : "memory");
-      if ((int32_t)(v - epoch) >= 0) { ok = true; break; }
-      if ((it & 63) == 0) {
-        uint64_t t;
-        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-        if (it == 0) t0 = t;
-        else if (t - t0 > timeout_ns) break;
-        else __nanosleep(200);
+  bool late = false;
+  for (uint32_t i = threadIdx.x; i < n; i += 32) late |= !flag_is_set(flags + which[i], epoch);
+  if (__any_sync(0xffffffffu, late)) {
+    uint64_t t0, t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
+    for (uint32_t i = threadIdx.x; i < n; i += 32) {
+      const uint32_t* flag = flags + which[i];
+      bool ok = false;
+      for (uint64_t it = 0; it < (1ull << 34); ++it) {
+        ok = flag_is_set(flag, epoch);
+        if (ok) break;
+        if ((it & 63) == 0) {
+          asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+          if (t - t0 > timeout_ns) break;
+          if (it) __nanosleep(200);
+        }
       }
+      if (!ok) missing = min(missing, i);
     }
-    if (!ok) missing = min(missing, i);
   }
   missing = __reduce_min_sync(0xffffffffu, missing);
   if (threadIdx.x == 0) {
