@@ -8,7 +8,7 @@ import torch
 
 from . import lib as _L
 from .lib import STATUS_BAD_OP, STATUS_OK, STATUS_TIMEOUT, cuda_lib
-from .table import LAUNCH_COUNT, CopyTable, SliceRef, device_index, dtype_code, make_spec, raw_stream
+from .table import LAUNCH_COUNT, CopyTable, SliceRef, dtype_code, make_spec
 
 FLAG_LAUNCH_COUNT = [0]  # set_flags / wait_flags kernels launched in this process
 
@@ -25,6 +25,10 @@ __all__ = [
     "STATUS_TIMEOUT",
     "STATUS_BAD_OP",
 ]
+
+
+def _handle(stream: torch.cuda.Stream | None, index: int) -> int:
+    return torch._C._cuda_getCurrentRawStream(index) if stream is None else stream.cuda_stream
 
 
 def _reachable(src: torch.Tensor, device: torch.device) -> None:
@@ -80,9 +84,8 @@ def local_copy(src: torch.Tensor, dst: torch.Tensor, stream: torch.cuda.Stream |
 
 def set_flags(addresses: torch.Tensor, epoch: int, stream: torch.cuda.Stream | None = None) -> None:
     """Store `epoch` (release, system scope) to every uint32 flag whose address is in `addresses` (int64, device)."""
-    device = addresses.device
-    rc = cuda_lib().etha_set_flags(addresses.data_ptr(), addresses.numel(), epoch & 0xFFFFFFFF, device_index(device),
-                                   raw_stream(stream, device))
+    index = addresses.get_device()
+    rc = cuda_lib().etha_set_flags(addresses.data_ptr(), addresses.numel(), epoch & 0xFFFFFFFF, index, _handle(stream, index))
     _L.check(rc, "set_flags")
     FLAG_LAUNCH_COUNT[0] += 1
 
@@ -100,9 +103,9 @@ def wait_flags(
     `status` (int32[2], device or pinned-mapped) receives `[STATUS_OK | STATUS_TIMEOUT, index of the
     first missing flag]`.  The wait gives up after `timeout_s`; the context stays usable.
     """
-    device = flags.device
+    index = flags.get_device()
     rc = cuda_lib().etha_wait_flags(flags.data_ptr(), which.data_ptr(), which.numel(), epoch & 0xFFFFFFFF, int(timeout_s * 1e9),
-                                    status.data_ptr(), device_index(device), raw_stream(stream, device))
+                                    status.data_ptr(), index, _handle(stream, index))
     if rc:
         _L.check(rc, "wait_flags")
     FLAG_LAUNCH_COUNT[0] += 1

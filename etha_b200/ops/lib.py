@@ -61,6 +61,8 @@ _lib = None
 def cuda_lib() -> C.CDLL:
     """Load (building first if the sources are newer) the CUDA library. Raises if it cannot be built."""
     global _lib
+    if _lib is not None:  # assigned once, when it is complete
+        return _lib
     with _lock:
         if _lib is not None:
             return _lib
