@@ -370,7 +370,9 @@ class P2PBatch:
     def send(self, stream: torch.cuda.Stream | None = None, ctas_per_sm: int = 2, bulk: bool = False,
              dma: bool | None = None) -> None:
         """Enqueue this rank's copies and the completion signal. Call `begin()` first.  `dma=False` keeps every copy
-        in the kernels for this transfer even when the batch was built with a DMA plan."""
+        in the kernels for this transfer even when the batch was built with a DMA plan.  `ctas_per_sm=1` leaves half
+        of every SM to other work while the LD/ST copy kernel runs; any other number lets it fill them.  Transfers of
+        one batch follow one another: do not enqueue the next on another stream without ordering the two."""
         if self.table is None:
             raise RuntimeError("build() first")
         if self._signals is None and self.table.empty:

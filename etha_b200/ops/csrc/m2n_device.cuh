@@ -269,7 +269,8 @@ __device__ __forceinline__ float round_through(float x) {
 // DRAM pages and the slowest SM sets the end.  A bare copy of 1 GiB with 16-byte units: fixed stride 5.7 to 6.0 TB/s (read
 // + written) with any block size, unroll or cache hint; tiles taken in order as SMs become free 6.7 to 6.9; one read
 // and four writes: 5.6 and 6.6.  Why not a counter in memory: the hardware's queue belongs to the launch, so two launches of one table (two
-// streams, a graph) share nothing and nothing has to be reset.  A CTA that takes tiles over pays its prologue (and the
+// streams, a graph) share no queue and nothing has to be reset.  Launches that signal share the table's count of finished
+// tiles, though, and have to follow one another (see `finish`).  A CTA that takes tiles over pays its prologue (and the
 // completion fence) once.
 //
 // `sync` is one 64-bit word to the kernels: finished tiles in the lower half, status bits in the upper one, so that the CTA
@@ -435,6 +436,8 @@ __device__ __forceinline__ uint32_t for_each_tile(TileSched* s, M2NOp* s_op, con
 // its system-scope release stores order them for the consumers too (release patterns are cumulative).  What a small table
 // of 592 CTAs pays for its signal: 13 us with a system-scope fence in every CTA, 5 us with a GPU-scope one there and a
 // system-scope fence before the release stores, 3 us as it stands.
+// The count belongs to the table: two signalling launches of one table that overlap would complete each other's count and
+// publish early.  They have to be ordered (one stream, or events); launches without signals do not touch it.
 // `done` holds failed and abandoned tiles too, so that the count closes and the next launch starts at 0.  Nothing is
 // published while the error word is set, in this launch or a later one: a flag never stands for data that was not
 // delivered, and consumers run into their own limit.

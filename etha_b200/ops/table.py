@@ -310,6 +310,7 @@ class CopyTable:
         return taken
 
     def finalize(self, sm_count: int | None = None) -> "CopyTable":
+        """Lay the table out and upload it.  `sm_count` is kept as an attribute; grids do not depend on it."""
         if self._final:
             return self
         if self.device.type == "cuda" and self.device.index is None:  # the table lives on one device from here on
@@ -376,6 +377,10 @@ class CopyTable:
         dma: bool | None = None,
     ) -> None:
         """Enqueue the table on `stream`. `signals`: int64 device tensor of flag addresses to publish `epoch` to.
+        Launches without signals may overlap on several streams; those with signals share the table's count of
+        finished tiles and must follow one another.
+        `ctas_per_sm`: 1 leaves half of every SM to other work while the 16-byte copy kernel runs; any other number
+        lets it fill the SMs, and the other kernels always do.
         `bulk`: TMA ring kernel instead of the LD/ST kernel for the 16-byte bit copies; `dma=False`: every copy by
         the kernels even if the table holds a DMA plan."""
         if not self._final:

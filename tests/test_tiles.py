@@ -66,7 +66,7 @@ def test_every_class_walks_all_tiles(bulk, repeat):
 
 @pytest.mark.gpu
 def test_two_streams_share_a_table():
-    """Launches of one table that overlap on the GPU take their tiles from queues of their own."""
+    """Launches of one table, without signals, that overlap on the GPU take their tiles from queues of their own."""
     dev = torch.device("cuda", 0)
     src = torch.arange(64 << 20, device=dev, dtype=torch.int32)
     dst = torch.zeros_like(src)
