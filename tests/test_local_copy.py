@@ -1,4 +1,4 @@
-"""`local_copy`: what it refuses, which device the launches go to, what they come after."""
+"""`local_copy`: what it refuses, which device the launches go to, what they come after; every kernel class through it."""
 
 from contextlib import nullcontext
 from types import SimpleNamespace
@@ -186,6 +186,36 @@ def test_other_streams_under_capture(forked):
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(dst, src)
+
+
+VIEWS = {  # kernel class -> (source, destination) shaped views of one buffer each
+    "fast run": lambda x, y: (x[:64].view(-1), y[:64].view(-1)),
+    "fast rows": lambda x, y: (x[:, 8:264], y[:, 16:272]),
+    "one element": lambda x, y: (x[3, 3:4], y[5, 7:8]),
+    "no element": lambda x, y: (x[:0], y[:0]),
+    "no dimension": lambda x, y: (x[2, 2], y[3, 3]),
+    "ragged": lambda x, y: (x[:, 1:258], y[:, 3:260]),
+    "ragged, two strided dims": lambda x, y: (x.view(16, 8, 272)[:, 1:7:2, 5:133], y.view(16, 8, 272)[:, ::3, 3:131]),
+    "transposing": lambda x, y: (x[:, :128], y[:, :128].t()),
+    "transposing, unaligned": lambda x, y: (x[1:100, 3:80], y[2:79, 5:104].t()),
+    "short rows": lambda x, y: (x[:, 1:4], y[:, 2:5]),
+    "element by element": lambda x, y: (x[:, ::2], y[:, 1::2]),
+    "broadcast source": lambda x, y: (x[:1].expand(128, 272), y),
+}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("view", VIEWS)
+@pytest.mark.parametrize("sdt,ddt", [(torch.bfloat16,) * 2, (torch.float32,) * 2, (torch.uint8,) * 2, (torch.float32, torch.bfloat16),
+                                     (torch.bfloat16, torch.float32), (torch.float16, torch.bfloat16)])
+def test_every_class_launched_alone(view, sdt, ddt):
+    x = torch.randint(-99, 99, (128, 272), device="cuda:0").to(sdt)
+    y = torch.randint(0, 9, (128, 272), device="cuda:0").to(ddt)
+    want = y.clone()
+    src, dst = VIEWS[view](x, y)
+    VIEWS[view](x, want)[1].copy_(src)
+    ops.local_copy(src, dst)
+    assert torch.equal(y, want)  # the rest of the destination included
 
 
 @pytest.mark.gpu

@@ -66,7 +66,6 @@ def test_typed_rows_equal_the_general_kernel(sdt, ddt, sizes, opnames):
             raise AssertionError
         outs = []
         for streaming in (True, False):
-            dsts = [_view(rows, cols, lead_d, ddt, 50).clone(memory_format=torch.preserve_format) for _ in range(2)]
             dsts = [torch.full((rows, cols + lead_d + 4), 7.0, dtype=ddt, device=DEV) for _ in range(2)]
             t = _table((rows, cols), srcs, [d[:, lead_d : lead_d + cols] for d in dsts], sizes, opnames, streaming)
             assert (t._packed[0][4] >> 12 == 1) == streaming
@@ -103,6 +102,43 @@ def test_special_values_pass_unchanged():
     dst = torch.zeros(5, 91, device=DEV)
     _run(_table((5, 89), [a, b], [dst[:, 1:90]], (2,), ("max",)))
     assert torch.equal(dst[:, 1:90], torch.maximum(a, b))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("sizes,opnames", [((2,), ("sum",)), ((3,), ("avg",)), ((2,), ("max",)), ((3,), ("min",)), ((2,), ("product",)), ((2, 2), ("max", "sum"))])
+def test_nan_and_infinity_through_collapses(dtype, sizes, opnames):
+    """Every pair of special values meets in some column; NaN wins over everything, as in torch."""
+    special = torch.tensor([float("nan"), float("inf"), float("-inf"), 0.0, -0.0, 1.5, torch.finfo(dtype).min, torch.finfo(dtype).max], device=DEV)
+    n, cols = 1, 8 * 8 + 25
+    for s in sizes:
+        n *= s
+    srcs = []
+    for i in range(n):
+        row = torch.full((cols,), 2.0, device=DEV)
+        row[:64] = special.repeat_interleave(8) if i % 2 else special.repeat(8)
+        srcs.append(row.to(dtype).repeat(3, 1 + 8 // n)[:, 1 : cols - 3])  # odd rows, not on a 16-byte boundary
+    steps = {"sum": torch.add, "avg": torch.add, "max": torch.maximum, "min": torch.minimum, "product": torch.mul}
+
+    def fold(values, name):
+        acc = values[0]
+        for v in values[1:]:
+            acc = steps[name](acc, v)
+        return acc / len(values) if name == "avg" else acc
+
+    want = [s.float() for s in srcs]
+    for size, name in zip(sizes, opnames):
+        want = [fold(want[k : k + size], name) for k in range(0, len(want), size)]
+    outs = []
+    for streaming in (True, False):
+        dst = torch.zeros(3, cols, dtype=dtype, device=DEV)
+        t = _table(tuple(srcs[0].shape), srcs, [dst[:, 3 : cols - 1]], sizes, opnames, streaming)
+        assert (t._packed[0][4] >> 12 == 1) == streaming
+        _run(t)
+        assert torch.equal(dst[:, 3 : cols - 1].isnan(), want[0].isnan())
+        torch.testing.assert_close(dst[:, 3 : cols - 1], want[0].to(dtype), rtol=0, atol=0, equal_nan=True)
+        outs.append(dst.view(torch.uint8))
+    assert torch.equal(*outs)
 
 
 @pytest.mark.parametrize("seed", range(40))
