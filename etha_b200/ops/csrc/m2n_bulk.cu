@@ -189,10 +189,8 @@ m2n_bulk_kernel(const __grid_constant__ M2NLaunch args) {
       }
       ++done;  // run or given up: see `finish`
       const Take take = sched_take(&ring.sched, phase, tile, args);
-      if (__any_sync(0xffffffffu, take == kGaveUp)) {
-        done += sched_abandon(&ring.sched, phase);
-        break;
-      }
+      __syncwarp();
+      if (gave_up(ring.sched.state, phase)) alive = false;
       phase ^= 1;
       if (!alive) done += take == kTile;  // taken over, but this CTA has stopped
       alive = alive && take == kTile;

@@ -311,13 +311,19 @@ __device__ __forceinline__ void sched_request(TileSched* s) {
                : "memory");
 }
 
-enum Take { kNoTile, kTile, kGaveUp };
+enum Take { kNoTile, kTile, kNoAnswer };
+constexpr uint32_t kAnswerSpins = 1u << 22;
 
-// one thread's bounded wait for the answer, and the tile in it
-__device__ __forceinline__ Take sched_answer(TileSched* s, uint32_t phase, uint32_t& tile) {
+// Every thread that asks waits for the answer, which names the next tile.  One that runs into the limit reports it, marks the
+// queue, and waits once more: no answer should arrive in the shared memory of a CTA that has ended.  All threads see the mark after
+// the barrier that the next request needs anyway, and stop together; a tile in the answer then counts as finished without being
+// run.  A mark per phase: a thread that is quick to give up on the next answer does not change what a slow one still has to read.
+// (With a voting barrier per tile instead, 1169.8 us for a sync that takes 1164.8; with the second wait in a place of its own, 5 more
+// registers and 121 us for ragged conversions that take 112.)
+__device__ __forceinline__ Take sched_take(TileSched* s, uint32_t phase, uint32_t& tile, const M2NLaunch& args) {
   const uint32_t bar = smem_addr(&s->bar);
   uint32_t ready = 0;
-  for (uint32_t spin = 0; spin < (1u << 22) && !ready; ++spin) {
+  for (uint32_t spin = 0; spin < 2 * kAnswerSpins && !ready; ++spin) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "mbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2;\n\t"
@@ -325,8 +331,12 @@ __device__ __forceinline__ Take sched_answer(TileSched* s, uint32_t phase, uint3
         : "=r"(ready)
         : "r"(bar), "r"(phase)
         : "memory");
+    if (spin == kAnswerSpins) {
+      report(args, M2N_TIMEOUT);
+      (phase ? s->state.w : s->state.z) = 1;
+    }
   }
-  if (!ready) return kGaveUp;
+  if (!ready) return kNoAnswer;
   uint32_t more;
   asm volatile(
       "{\n\t.reg .pred p;\n\t.reg .b128 h;\n\t"
@@ -342,24 +352,8 @@ __device__ __forceinline__ Take sched_answer(TileSched* s, uint32_t phase, uint3
   return more ? kTile : kNoTile;
 }
 
-// Every thread that asks waits for the answer.  One that gives up reports it and marks the queue: all threads see the mark
-// after the barrier that the next request needs anyway, and stop together.  A mark per phase: a thread that is quick to give up
-// on the next answer does not change what a slow one still has to read.  (With a voting barrier per tile instead, 1169.8 us for a sync that takes 1164.8.)
-__device__ __forceinline__ Take sched_take(TileSched* s, uint32_t phase, uint32_t& tile, const M2NLaunch& args) {
-  const Take take = sched_answer(s, phase, tile);
-  if (take == kGaveUp) {
-    report(args, M2N_TIMEOUT);
-    (phase ? s->state.w : s->state.z) = 1;
-  }
-  return take;
-}
-
-// After a thread has given up: waits once more, so that no answer arrives in the shared memory of a CTA that has ended, and
-// returns the number of tiles (0 or 1) that the answer took out of the queue.  They are counted as finished without being run.
-__device__ __noinline__ uint32_t sched_abandon(TileSched* s, uint32_t phase) {
-  uint32_t tile;
-  return sched_answer(s, phase, tile) == kTile;
-}
+// whether a thread has given up in `phase`; the threads that asked have been synchronised since
+__device__ __forceinline__ bool gave_up(const uint4& state, uint32_t phase) { return phase ? state.w : state.z; }
 
 // one warp loads the op that owns `tile` (looked up 32 ways at a time) into shared memory; returns its tiles
 __device__ __forceinline__ uint2 load_op(const M2NLaunch& args, uint32_t tile, M2NOp* s_op) {
@@ -411,24 +405,24 @@ __device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepc
 template <bool CHUNKS = false, typename Body>
 __device__ __forceinline__ uint32_t for_each_tile(TileSched* s, M2NOp* s_op, const M2NLaunch& args, Body&& body) {
   sched_init(s);
-  uint32_t tile = blockIdx.x, done = 0, phase = 0;
+  uint32_t tile = blockIdx.x, taken = 1, phase = 0;
   Take take;
   uint4 state = s->state;
   do {
     if (threadIdx.x == 0) sched_request(s);
     const uint32_t first = sched_locate(s, state, args, tile, s_op);
-    if (!done) after_previous_kernel();
+    if (taken == 1) after_previous_kernel();
     const M2NOp& op = *s_op;
     const uint32_t base = (tile - first) * op.tile_units;
     body(op, base, min(CHUNKS ? op.chunks : op.total_units, base + op.tile_units));
-    ++done;
     take = sched_take(s, phase, tile, args);
     __syncthreads();
     state = s->state;
-    if (phase ? state.w : state.z) return done + sched_abandon(s, phase);
+    if (take != kTile) return taken;
+    ++taken;
+    if (gave_up(state, phase)) return taken;
     phase ^= 1;
-  } while (take == kTile);
-  return done;
+  } while (true);
 }
 
 // The CTA that finishes the last tile publishes `epoch` to every flag with system-scope release ordering.  Each CTA

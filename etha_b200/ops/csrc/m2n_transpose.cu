@@ -12,6 +12,8 @@
 // [16384, 8192] on one GPU, TB/s read + written, general kernel -> here: bf16 0.40 -> 5.27, fp32 0.79 -> 4.42, fp32 -> bf16
 // 0.68 -> 4.23, bf16 with an odd width 0.44 -> 2.60, odd height 0.40 -> 1.83, both 0.44 -> 1.33; 16 wide (1/4 of a block's
 // rows used) 0.47 -> 1.59, 8 wide 0.41 -> 0.82.  Five CTAs per SM: four give 5.06 and 4.22, six 4.51 and 4.20.
+// At five (48 registers) every instance spills 32 to 64 bytes a thread; at four (64) five of the eight spill nothing, which does
+// not make up for the loads in flight.
 #include <cuda_runtime.h>
 
 #include <cstdio>

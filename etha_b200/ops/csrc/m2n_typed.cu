@@ -112,7 +112,8 @@ m2n_typed_kernel(const __grid_constant__ M2NLaunch args) {
 // first value is used, which is what the general kernel lacks: it reads one source after the other.  128 MiB per source on
 // one GPU, TB/s read + written, general kernel -> here: sum of 3 bf16 2.4 -> 5.2, 8 bf16 3.9 -> 6.3, 8 fp32 2.9 -> 6.6, 2 x 2
 // bf16 1.8 -> 4.7, 2 x 4 fp32 1.9 -> 5.8, maximum of 8 bf16 (bound by the comparisons) 3.2 -> 3.6.  Two CTAs per SM: three
-// spill and reach 5.0, 6.0, 4.3, 3.5, 3.3.
+// spill and reach 5.0, 6.0, 4.3, 3.5, 3.3.  Two levels keep a group and the total: those instances spill 52 to 108 bytes a thread at
+// two CTAs as well.
 constexpr int kSlots = 4;
 
 template <int SDT, int DDT, bool TWO, int U>
