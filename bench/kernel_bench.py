@@ -3,7 +3,7 @@
 
 Cases: `copy` (contiguous), `rows` (Shard(0) shard cut into 4 column blocks, the o_proj/down_proj
 pattern), `cvt` (fp32 -> bf16), `reduce2` / `reduce4` (Partial collapse of 2 / 4 bf16 sources),
-`fanout4` (one read, four destinations).  Buffers are larger than L2; timing uses CUDA events around
+`fanout4` (one read, four destinations), `ragged` (801 of 1601 columns), `transpose` ([N, 8192]).  Buffers are larger than L2; timing uses CUDA events around
 each launch after warm-up.  Prints one JSON line per case with achieved bytes/s against the measured
 copy bandwidth in MEASURED_PEAKS.json (fallback 6.65 TB/s).
 
@@ -74,6 +74,18 @@ def build_case(case: str, mb: int, dev, tile_kb: int, streaming: bool = True):
         keep += [src] + dsts
         traffic = 5 * src.numel() * 2
         check = lambda: all(torch.equal(d, src) for d in dsts)
+    elif case == "ragged":
+        src = torch.randn(mb * 1024 * 1024 // 3202, 1601, device=dev).to(torch.bfloat16)[:, :801]
+        dst = torch.empty(src.shape, dtype=src.dtype, device=dev)
+        t.add_copy(src, dst)
+        traffic = 2 * dst.numel() * 2
+        check = lambda: torch.equal(src, dst)
+    elif case == "transpose":
+        src = torch.randn(2 * n_rows // 4, 8192, device=dev).to(torch.bfloat16)
+        dst = torch.empty(8192, src.shape[0], dtype=src.dtype, device=dev)
+        t.add_copy(src.t(), dst)
+        traffic = 2 * dst.numel() * 2
+        check = lambda: torch.equal(src.t(), dst)
     else:
         raise ValueError(case)
     t.finalize()
@@ -94,7 +106,7 @@ def main():
     dev = torch.device("cuda", 0)
     torch.cuda.set_device(dev)
     peak, how = peak_gbs()
-    cases = ["copy", "rows", "cvt", "reduce2", "reduce4", "fanout4"] if args.case == "all" else [args.case]
+    cases = ["copy", "rows", "cvt", "reduce2", "reduce4", "fanout4", "ragged", "transpose"] if args.case == "all" else [args.case]
     for case in cases:
         table, traffic, check, keep = build_case(case, args.mb, dev, args.tile_kb, bool(args.streaming))
         for _ in range(args.warmup):

@@ -247,8 +247,8 @@ __device__ __forceinline__ bool dispatch_typed(const M2NOp& op, uint32_t base, u
 
 // Fast class: 16-byte bit copies whose box is one run or rows of a matrix (the bulk of a weight sync).  Bound by HBM (or
 // NVLink): 4 x 512 threads per SM at 32 registers, two 16-byte loads each before the first store, tiles of one such trip
-// (16 KiB).  1 GiB on one GPU, read + written: contiguous 6.72 TB/s, 2 KiB rows out of 8 KiB ones 6.45, one source and four
-// destinations 6.51 (2 x 512 threads with four loads and a fixed stride of 64 KiB tiles: 5.52, 5.79, 5.37).  With 76 bytes of
+// (16 KiB).  1 GiB on one GPU, read + written: contiguous 6.71 TB/s, 2 KiB rows out of 8 KiB ones 6.46, one source and four
+// destinations 6.52 (2 x 512 threads with four loads and a fixed stride of 64 KiB tiles: 5.52, 5.79, 5.37).  With 76 bytes of
 // spills per thread the same kernel falls to 5.97, so full trips carry no per-unit predicate.
 constexpr int kFastThreads = 512;
 constexpr int kFastCtas = 4;

@@ -9,8 +9,9 @@
 // their shape, and the 8 x 4 words that a warp collects at once lie in 32 different banks.
 // A side that is not 16-byte aligned is moved element by element on that side; a block whose destination is not aligned
 // is swizzled by w ^ a % 32 instead, since a warp then reads 32 consecutive a of one b.
-// [16384, 8192] on one GPU, TB/s read + written, general kernel -> here: bf16 0.40 -> 5.27, fp32 0.79 -> 4.42, fp32 -> bf16
-// 0.68 -> 4.23, bf16 with an odd width 0.44 -> 2.60, odd height 0.40 -> 1.83, both 0.44 -> 1.33; 16 wide (1/4 of a block's
+// [16384, 8192] on one GPU, TB/s read + written, general kernel -> here: bf16 0.40 -> 5.0 to 5.3, fp32 0.79 -> 4.4, fp32 -> bf16
+// 0.68 -> 4.1, bf16 with an odd width 0.44 -> 2.5, odd height 0.40 -> 1.8, both 0.44 -> 1.3 ([65536, 8192] bf16: 5.54, with 71 % of the
+// issue slots busy and DRAM at 60 % of its peak); 16 wide (1/4 of a block's
 // rows used) 0.47 -> 1.59, 8 wide 0.41 -> 0.82.  Five CTAs per SM: four give 5.06 and 4.22, six 4.51 and 4.20.
 // At five (48 registers) every instance spills 32 to 64 bytes a thread; at four (64) five of the eight spill nothing, which does
 // not make up for the loads in flight.

@@ -6,8 +6,8 @@
 // needs for its `kUnits` units (all sources of all units, 128 bytes per thread) is issued before the first value
 // is used, so that a Partial collapse whose other contributors live on peer GPUs keeps enough bytes in flight to
 // cover the NVLink round trip.  Two 256-thread CTAs per SM (up to 128 registers per thread: no spills); tiles are taken
-// dynamically (see TileSched).  1 GiB of bf16 results on one GPU, read + written: fp32 -> bf16 6.79 TB/s, two bf16 sources
-// 6.83, four 6.72 (with fixed shares of 64 KiB tiles 6.57, 5.90 and 6.19).
+// dynamically (see TileSched).  1 GiB of bf16 results on one GPU, read + written: fp32 -> bf16 6.88 TB/s, two bf16 sources
+// 6.90, four 6.76 (with fixed shares of 64 KiB tiles 6.57, 5.90 and 6.19).
 // Arithmetic is the same as the general kernel's: fp32 accumulation in source order, "avg" divides by the
 // number of sources, one rounding to the source dtype when the destination dtype differs, then conversion.
 //
@@ -110,8 +110,8 @@ m2n_typed_kernel(const __grid_constant__ M2NLaunch args) {
 // Collapses without an instance of their own (3 or 5 to 8 sources, two levels, the two 16-bit types mixed): one kernel per
 // dtype pair, for one and for two levels.  The sources are read four at a time, all loads of the four issued before the
 // first value is used, which is what the general kernel lacks: it reads one source after the other.  128 MiB per source on
-// one GPU, TB/s read + written, general kernel -> here: sum of 3 bf16 2.4 -> 5.2, 8 bf16 3.9 -> 6.3, 8 fp32 2.9 -> 6.6, 2 x 2
-// bf16 1.8 -> 4.7, 2 x 4 fp32 1.9 -> 5.8, maximum of 8 bf16 (bound by the comparisons) 3.2 -> 3.6.  Two CTAs per SM: three
+// one GPU, TB/s read + written, general kernel -> here: sum of 3 bf16 2.4 -> 5.1, 8 bf16 3.9 -> 6.1, 8 fp32 2.9 -> 6.4, 2 x 2
+// bf16 1.8 -> 4.5, 2 x 4 fp32 1.9 -> 5.6, maximum of 8 bf16 (bound by the comparisons) 3.2 -> 3.6.  Two CTAs per SM: three
 // spill and reach 5.0, 6.0, 4.3, 3.5, 3.3.  Two levels keep a group and the total: those instances spill 52 to 108 bytes a thread at
 // two CTAs as well.
 constexpr int kSlots = 4;
