@@ -18,7 +18,7 @@
 //
 // 1 GiB on one GPU, read + written: contiguous 6.63 TB/s, 2 KiB rows out of 8 KiB ones 6.52, one source and four
 // destinations 6.50 (one warp for both directions and a fixed stride of tiles: 6.00, 5.42, 5.67).  Six stages of 32 KiB,
-// on a box where they gave 6.55 / 6.46 / 6.46: 12 x 16 KiB gives 6.48 / 6.19 / 6.46, 3 x 32 KiB 6.48 / 6.40 / 6.42.
+// on a GPU where they gave 6.55 / 6.46 / 6.46: 12 x 16 KiB gives 6.48 / 6.19 / 6.46, 3 x 32 KiB 6.48 / 6.40 / 6.42.
 #include <cuda_runtime.h>
 #include <stdint.h>
 

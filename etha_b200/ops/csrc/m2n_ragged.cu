@@ -27,7 +27,7 @@ constexpr int kRawChunk = M2N_RAGGED_BYTES;
 
 // CTAs per SM and chunks in flight per thread, as far as the registers go without spills.  Measured on one GPU (read +
 // written): 131072 rows of 801 of 1601 bf16 columns 5.03 TB/s with 5 CTAs and two chunks (6 x 1: 4.80, 3 x 3: 3.87; chunks of 16 bytes: 4.63
-// at best; 5.45 with 335000 rows; other boxes 4.8), the same columns fp32 -> bf16 5.6 (general kernel, element by element: 0.66 and 1.03).
+// at best; 5.45 with 335000 rows; another GPU 4.8), the same columns fp32 -> bf16 5.6 (general kernel, element by element: 0.66 and 1.03).
 template <int SDT, bool REDUCE>
 constexpr int kRaggedCtas = SDT == M2N_RAW ? 5 : (REDUCE ? 2 : 3);
 constexpr int kRaggedUnroll = 2;
